@@ -241,9 +241,9 @@ constexpr size_t rawTileBytes() {
   return (sizeof(RawTile<T, BS>) + 15) & ~size_t(15);
 }
 
-template <typename T, int BS>
+template <typename T, int BS, int ZG>
 constexpr size_t colorSmemBytes() {
-  return rawTileBytes<T, BS>() + 2 * sizeof(float) * ColorSweep<T, BS>::PLX * ColorSweep<T, BS>::NW;
+  return rawTileBytes<T, BS>() + 2 * sizeof(float) * ColorSweep<T, BS>::PLX * ColorSweep<T, BS>::NW * ZG;
 }
 
 template <typename T>
@@ -253,12 +253,26 @@ __device__ __forceinline__ float ldval(const T *p) {
 
 // FK: the stencil, fixed at compile time.  0 = any kind in the reference's
 // operation order (computeStrip); K_MCF / K_JACOBI = the fast forms, plus
-// FK_CLAMP when the result is clamped to [0,1].
-template <typename T, int BS, int FK>
-__global__ void __launch_bounds__(ColorSweep<T, BS>::NT, 2) kSweepColor(ColorArgs a) {
+// FK_CLAMP when the result is clamped to [0,1]; K_MCF | FK_EXACT = MCF in the
+// reference's order on packed operations (mcfExactStrip).
+//
+// ZG z-groups of NT threads share the staged block, each marching BS / ZG of its planes
+// (zGroups has the rule and its measurements).  A small pass is bound by the latency of one
+// block, not by bandwidth or issue: with one group, 64 threads march a 16^3 block.
+//
+// The passes of a call are launched with programmatic serialization: a pass's CTAs look up
+// their blocks and neighbours and prepare their copies while the previous pass drains, and
+// wait for its writes (griddepcontrol.wait) before the first copy.  Only warp 0 waits: what
+// the other warps read arrives through its copies, and what they write comes after.  The
+// trigger stands at the end of a CTA: at its start, the next pass's CTAs took places on the
+// SMs early and unevenly (216 blocks: 13.4 -> 16.9 us; at the end 11.2 us).
+template <typename T, int BS, int FK, int ZG>
+__global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, ColorSweep<T, BS>::NT *ZG <= 256 ? 2 : 1)
+    kSweepColor(ColorArgs a) {
   using C = ColorSweep<T, BS>;
   using V4 = typename Vec4T<T>::V;
   constexpr int RS = C::RS, PL = C::PL, PLX = C::PLX, CZ = C::CZ, NCH = C::NCH;
+  constexpr int PZ = BS / ZG;  // planes of a z-group
   extern __shared__ __align__(128) unsigned char dynSmem[];
   RawTile<T, BS> &t = *reinterpret_cast<RawTile<T, BS> *>(dynSmem);
   __shared__ int nbs[27];
@@ -285,27 +299,41 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT, 2) kSweepColor(ColorArg
   }
   __syncthreads();
   if (tid < 32) {
-    // warp 0, chunk by chunk: announce the chunk's bytes, then issue its copies lane-parallel
-    for (int k = 0; k < NCH; k++) {
-      void *d = nullptr;
-      const void *s = nullptr;
-      uint32_t b = 0;
-      const bool has = tid < C::NCC && tileCopy<T, BS>(k, tid, nbs, a, t, d, s, b);
-      uint32_t tot = has ? b : 0;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    // warp 0, lane-parallel over a chunk's copies: announce the chunk's bytes, then issue.
+    // A small pass prepares all chunks while the previous pass drains; a 32^3 block, whose
+    // passes are bound by throughput, issues each chunk as soon as it is known (preparing
+    // all four first costs Jacobi 1.4% on 498 M voxels).
+    constexpr bool PRE = BS == 16;
+    void *d[NCH];
+    const void *src[NCH];
+    uint32_t b[NCH];
+    auto prepare = [&](int k) {
+      const bool has = tid < C::NCC && tileCopy<T, BS>(k, tid, nbs, a, t, d[k], src[k], b[k]);
+      if (!has) b[k] = 0;
+      const uint32_t tot = __reduce_add_sync(0xffffffffu, b[k]);
       if (tid == 0) mbarExpectTx(&bar[k], tot);
       __syncwarp();
-      if (has) bulkG2S(d, s, b, &bar[k]);
+    };
+    if constexpr (PRE) {
+#pragma unroll
+      for (int k = 0; k < NCH; k++) prepare(k);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < NCH; k++) {
+      if constexpr (!PRE) prepare(k);
+      if (b[k]) bulkG2S(d[k], src[k], b[k], &bar[k]);
     }
   }
 
   const int ownSlot = nbs[13];
-  const int lane = tid & 31, warp = tid >> 5;
-  const int ty = tid / C::SPR, tx = (tid % C::SPR) * 4;  // this thread's strip
+  const int lane = tid & 31, zg = tid / C::NT, gt = tid % C::NT;
+  const int warp = gt >> 5;                              // warp within the z-group
+  const int zFirst = zg * PZ;                            // first plane of the z-group
+  const int ty = gt / C::SPR, tx = (gt % C::SPR) * 4;    // this thread's strip
   const int y0w = warp * C::RPW;                          // first row of this warp
   const int tyl = ty - y0w;                               // row inside the warp
-  float *wring = reinterpret_cast<float *>(dynSmem + rawTileBytes<T, BS>()) + warp * 2 * PLX;
+  float *wring = reinterpret_cast<float *>(dynSmem + rawTileBytes<T, BS>()) + (tid >> 5) * 2 * PLX;
   float emptyF;
   {
     T e;
@@ -430,7 +458,9 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT, 2) kSweepColor(ColorArg
 
   // ---- warp ring slot -> this thread's plane (rows y-1..y+1, x-1..x+4) ----
   constexpr int FKK = FK & ~FK_CLAMP;
-  using PW = std::conditional_t<FKK == K_MCF, PlaneMcf, std::conditional_t<FKK == K_JACOBI, PlaneJac, PlaneRaw>>;
+  using PW = std::conditional_t<
+      FKK == K_MCF, PlaneMcf,
+      std::conditional_t<FKK == K_JACOBI, PlaneJac, std::conditional_t<FKK == (K_MCF | FK_EXACT), PlaneMcfX, PlaneRaw>>>;
   const int winOff = tyl * RS + tx + 3;
   auto window = [&](const float *pl, PW &w) { loadPlane<RS>(pl + winOff, w); };
 
@@ -447,6 +477,7 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT, 2) kSweepColor(ColorArg
     float out[4];
     constexpr bool CL = (FK & FK_CLAMP) != 0;
     if constexpr (FKK == K_MCF) mcfFastStrip<CL>(Wm, W0, Wp, a.p.dt, out);
+    else if constexpr (FKK == (K_MCF | FK_EXACT)) mcfExactStrip(Wm, W0, Wp, a.p.dt, a.p.negZero, a.p.constr01, out);
     else if constexpr (FKK == K_JACOBI) jacobiFastStrip<CL>(Wm, W0, Wp, a.p.dt, out);
     else computeStrip(Wm.w, W0.w, Wp.w, a.p, out);
     const V4 pk = pack4<T>(out);
@@ -482,45 +513,79 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT, 2) kSweepColor(ColorArg
   };
   using Interior = std::integral_constant<int, 0>;
 
-  // planes -1, 0, 1 into the windows (warp-local ring slots 0/1)
-  fillZ(-1, wring);
-  fillInterior(0, wring + PLX);
-  __syncwarp();
-  window(wring, Wa);
-  window(wring + PLX, Wb);
-  __syncwarp();
-  fillInterior(1, wring);
-  loadRaw(2);
-  __syncwarp();
-  window(wring, Wc);
-  __syncwarp();
-  // The window roles rotate every plane: (a,b,c) -> (b,c,a).  The main loop runs
-  // the planes z whose planes z+2 and z+3 are interior, three at a time; the
-  // last planes follow with their kinds known at compile time.
-  constexpr int MAIN = 3 * ((BS - 3) / 3);
+  // The loop in one copy: the exact form is bound by instruction fetch when its planes are
+  // unrolled (16^3 blocks, 1000 a pass: 32.6 us unrolled, generic scalar form; 21.8 us rolled
+  // and packed), and a z-group has few planes.
+  constexpr bool ROLL = ZG > 1 || FKK == (K_MCF | FK_EXACT);
+  if constexpr (!ROLL) {
+    // planes -1, 0, 1 into the windows (warp-local ring slots 0/1)
+    fillZ(-1, wring);
+    fillInterior(0, wring + PLX);
+    __syncwarp();
+    window(wring, Wa);
+    window(wring + PLX, Wb);
+    __syncwarp();
+    fillInterior(1, wring);
+    loadRaw(2);
+    __syncwarp();
+    window(wring, Wc);
+    __syncwarp();
+    // The window roles rotate every plane: (a,b,c) -> (b,c,a).  The main loop runs
+    // the planes z whose planes z+2 and z+3 are interior, three at a time; the
+    // last planes follow with their kinds known at compile time.
+    constexpr int MAIN = 3 * ((BS - 3) / 3);
 #pragma unroll 1
-  for (int z = 0; z < MAIN; z += 3) {
-    step(Interior{}, z, Wa, Wb, Wc);
-    step(Interior{}, z + 1, Wb, Wc, Wa);
-    step(Interior{}, z + 2, Wc, Wa, Wb);
-  }
-  static_assert(BS - MAIN >= 3 && BS - MAIN <= 5, "tail of 3..5 planes");
-  auto tail = [&](auto zc) {
-    constexpr int z = decltype(zc)::value;
-    if constexpr (z < BS) {
-      constexpr int K = z + 3 < BS ? 0 : z + 2 < BS ? 3 : (z + 2 == BS ? 1 : 2);
-      using KT = std::integral_constant<int, K>;
-      constexpr int r = (z - MAIN) % 3;
-      if constexpr (r == 0) step(KT{}, z, Wa, Wb, Wc);
-      else if constexpr (r == 1) step(KT{}, z, Wb, Wc, Wa);
-      else step(KT{}, z, Wc, Wa, Wb);
+    for (int z = 0; z < MAIN; z += 3) {
+      step(Interior{}, z, Wa, Wb, Wc);
+      step(Interior{}, z + 1, Wb, Wc, Wa);
+      step(Interior{}, z + 2, Wc, Wa, Wb);
     }
-  };
-  tail(std::integral_constant<int, MAIN>{});
-  tail(std::integral_constant<int, MAIN + 1>{});
-  tail(std::integral_constant<int, MAIN + 2>{});
-  tail(std::integral_constant<int, MAIN + 3>{});
-  tail(std::integral_constant<int, MAIN + 4>{});
+    static_assert(BS - MAIN >= 3 && BS - MAIN <= 5, "tail of 3..5 planes");
+    auto tail = [&](auto zc) {
+      constexpr int z = decltype(zc)::value;
+      if constexpr (z < BS) {
+        constexpr int K = z + 3 < BS ? 0 : z + 2 < BS ? 3 : (z + 2 == BS ? 1 : 2);
+        using KT = std::integral_constant<int, K>;
+        constexpr int r = (z - MAIN) % 3;
+        if constexpr (r == 0) step(KT{}, z, Wa, Wb, Wc);
+        else if constexpr (r == 1) step(KT{}, z, Wb, Wc, Wa);
+        else step(KT{}, z, Wc, Wa, Wb);
+      }
+    };
+    tail(std::integral_constant<int, MAIN>{});
+    tail(std::integral_constant<int, MAIN + 1>{});
+    tail(std::integral_constant<int, MAIN + 2>{});
+    tail(std::integral_constant<int, MAIN + 3>{});
+    tail(std::integral_constant<int, MAIN + 4>{});
+  } else {
+    // plane p = -1 .. BS into a ring slot
+    auto stagePlane = [&](int p, float *slot) {
+      if (p < 0 || p >= BS) fillZ(p, slot);
+      else fillInterior(p, slot);
+    };
+    stagePlane(zFirst - 1, wring);
+    fillInterior(zFirst, wring + PLX);
+    __syncwarp();
+    window(wring, Wa);
+    window(wring + PLX, Wb);
+    __syncwarp();
+    stagePlane(zFirst + 1, wring);
+    __syncwarp();
+    window(wring, Wc);
+    __syncwarp();
+#pragma unroll 1
+    for (int i = 0; i < PZ; i++) {
+      float *slot = wring + ((i + 1) & 1) * PLX;
+      const bool more = i + 1 < PZ;
+      if (more) stagePlane(zFirst + i + 2, slot);
+      __syncwarp();
+      emit(zFirst + i, Wa, Wb, Wc);
+      Wa = Wb;
+      Wb = Wc;
+      if (more) window(slot, Wc);
+    }
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // let the next pass in
   if (timedOut) {
     atomicOr(a.status, 1);
     for (int k = 0; k < NCH; k++) waitChunk(&bar[k]);  // no copy may land after exit
@@ -542,6 +607,75 @@ __global__ void kExtractFaces(const T *__restrict__ pay, int64_t nAct, T *__rest
     const int ky = y == 0 ? 0 : 1;
     corners[(s * 4 + 0 + 2 * ky) * BS + z] = row[0];
     corners[(s * 4 + 1 + 2 * ky) * BS + z] = row[BS - 1];
+  }
+}
+
+// the stencil forms of kSweepColor: any kind in the reference's operation order, the fast
+// forms with and without the clamp, and MCF in the reference's order
+enum { kKernGeneric, kKernMcf, kKernMcfClamp, kKernJacobi, kKernJacobiClamp, kKernMcfExact };
+
+// z-groups per CTA of a pass of n blocks.  A pass is as long as one block takes while its
+// CTAs fit the chip at once (152 SMs), and more groups shorten a block; they cost every
+// group two more planes to stage, so a pass of several waves takes fewer.  Measured, us a
+// pass for 1 / 2 / 4 groups (FP32, 16^3 blocks): exact MCF 11.0 / 7.9 / 6.6 at 64 blocks,
+// 12.2 / 9.7 / 8.3 at 216, 15.4 / 12.8 / 16.3 at 512, 21.8 / 23.3 / 30.6 at 1000; fast MCF
+// 6.9 / 6.8 / 6.1 at 64, 11.6 / 11.0 / 14.9 at 512; fast Jacobi 5.7 / 5.7 / 5.3 at 64.
+// Two 4-group CTAs or four 2-group CTAs (registers) share an SM.  On 32^3 blocks the exact
+// form takes two groups up to one block per SM (24.2 -> 19.2 us, FP16, 64 blocks) and,
+// with FP32 storage, whose 145 KB of staging leave one CTA per SM, always (96.8 -> 80.9 us
+// at 512 blocks); the fast forms are not faster with two.
+template <typename T, int BS>
+static int zGroups(int n, int ki) {
+  constexpr int kSm = 152;
+  if constexpr (BS == 16) {
+    if (n <= 2 * kSm) return 4;
+    return ki == kKernMcfExact && n <= 4 * kSm ? 2 : 1;
+  } else {
+    return ki == kKernMcfExact && (sizeof(T) == 4 || n <= kSm) ? 2 : 1;
+  }
+}
+
+template <typename T, int BS, int FK, int ZG>
+static cudaError_t launchPassT(const ColorArgs &a, unsigned blocks, cudaStream_t st) {
+  const auto kern = kSweepColor<T, BS, FK, ZG>;
+  constexpr size_t smem = colorSmemBytes<T, BS, ZG>();
+  static bool attrSet = false;
+  if (!attrSet) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attrSet = true;
+  }
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(ColorSweep<T, BS>::NT * ZG);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+template <typename T, int BS>
+static cudaError_t launchPass(const ColorArgs &a, int ki, int zg, unsigned blocks, cudaStream_t st) {
+  constexpr int ZS = BS == 16 ? 4 : 1;  // the small passes' groups (generic and fast forms)
+  switch (ki) {
+    case kKernMcf: return zg > 1 ? launchPassT<T, BS, K_MCF, ZS>(a, blocks, st) : launchPassT<T, BS, K_MCF, 1>(a, blocks, st);
+    case kKernMcfClamp:
+      return zg > 1 ? launchPassT<T, BS, K_MCF | FK_CLAMP, ZS>(a, blocks, st)
+                    : launchPassT<T, BS, K_MCF | FK_CLAMP, 1>(a, blocks, st);
+    case kKernJacobi:
+      return zg > 1 ? launchPassT<T, BS, K_JACOBI, ZS>(a, blocks, st) : launchPassT<T, BS, K_JACOBI, 1>(a, blocks, st);
+    case kKernJacobiClamp:
+      return zg > 1 ? launchPassT<T, BS, K_JACOBI | FK_CLAMP, ZS>(a, blocks, st)
+                    : launchPassT<T, BS, K_JACOBI | FK_CLAMP, 1>(a, blocks, st);
+    case kKernMcfExact:
+      if (zg == ZS && ZS > 1) return launchPassT<T, BS, K_MCF | FK_EXACT, ZS>(a, blocks, st);
+      return zg == 2 ? launchPassT<T, BS, K_MCF | FK_EXACT, 2>(a, blocks, st)
+                     : launchPassT<T, BS, K_MCF | FK_EXACT, 1>(a, blocks, st);
+    default: return zg > 1 ? launchPassT<T, BS, 0, ZS>(a, blocks, st) : launchPassT<T, BS, 0, 1>(a, blocks, st);
   }
 }
 
@@ -571,21 +705,12 @@ static int runColorT(msbg_gpu_ctx *ctx, Channel &c, bool exact, bool color8, int
   a.emptyValue = 0.0f;
   a.status = ctx->dStatus;
   a.p = p;
-  constexpr size_t smem = colorSmemBytes<T, BS>();
-  void (*const kerns[5])(ColorArgs) = {kSweepColor<T, BS, 0>, kSweepColor<T, BS, K_MCF>,
-                                       kSweepColor<T, BS, K_MCF | FK_CLAMP>, kSweepColor<T, BS, K_JACOBI>,
-                                       kSweepColor<T, BS, K_JACOBI | FK_CLAMP>};
-  int ki = 0;  // the exact variant and the other kinds: the generic kernel
-  if (!exact && p.kind == K_MCF) ki = p.constr01 ? 2 : 1;
-  else if (!exact && p.kind == K_JACOBI) ki = p.constr01 ? 4 : 3;
-  const auto kern = kerns[ki];
-  static bool attrSet[5] = {false, false, false, false, false};
-  if (!attrSet[ki]) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attrSet[ki] = true;
-  }
+  int ki = kKernGeneric;
+  if (p.kind == K_MCF) ki = exact ? kKernMcfExact : p.constr01 ? kKernMcfClamp : kKernMcf;
+  else if (p.kind == K_JACOBI && !exact) ki = p.constr01 ? kKernJacobiClamp : kKernJacobi;
   static const int rbOrder[2][4] = {{1, 2, 4, 7}, {0, 3, 5, 6}};
-  constexpr int NT = ColorSweep<T, BS>::NT;
+  int zgOf[8];
+  for (int c8 = 0; c8 < 8; c8++) zgOf[c8] = zGroups<T, BS>(cs[c8 + 1] - cs[c8], ki);
   int nLaunch = 0;
   for (int pass = 0; pass < 8; pass++) nLaunch += cs[pass + 1] > cs[pass];
   nLaunch *= nIter;
@@ -597,8 +722,7 @@ static int runColorT(msbg_gpu_ctx *ctx, Channel &c, bool exact, bool color8, int
         const int cnt = cs[col + 1] - cs[col];
         if (cnt <= 0) continue;
         a.bids = bids + cs[col];
-        kern<<<(unsigned)cnt, NT, smem, st>>>(a);
-        if (cudaGetLastError() != cudaSuccess) return MSBG_GPU_ERR_CUDA;
+        if (launchPass<T, BS>(a, ki, zgOf[col], (unsigned)cnt, st) != cudaSuccess) return MSBG_GPU_ERR_CUDA;
       }
     }
     return MSBG_GPU_OK;
@@ -620,7 +744,7 @@ static int runColorT(msbg_gpu_ctx *ctx, Channel &c, bool exact, bool color8, int
     const unsigned char *b = reinterpret_cast<const unsigned char *>(&v);
     key.insert(key.end(), b, b + sizeof(v));
   };
-  put(reinterpret_cast<const void *>(kern)); put(bids); put(a.slot); put(a.payload); put(a.faces); put(a.corners);
+  put(reinterpret_cast<const void *>(&runColorT<T, BS>)); put(ki); put(bids); put(a.slot); put(a.payload); put(a.faces); put(a.corners);
   put(a.nbx); put(a.nby); put(a.nbz); put(a.emptyValue); put(a.status);
   put(p.kind); put(p.constr01); put(p.dt); put(p.anisAlpha); put(nIter); put(color8);
   for (int i = 0; i < 9; i++) put(cs[i]);

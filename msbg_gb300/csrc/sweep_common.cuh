@@ -7,11 +7,14 @@
 namespace msbg {
 
 enum { K_MCF = 4, K_JACOBI = 17, K_PM_JACOBI = 15, K_PM = 14, K_DIFF = 3, K_LAPL = 1 };
-enum { FK_CLAMP = 256 };  // sweep kernel flag: results clamped to [0,1]
+// sweep kernel flags: results clamped to [0,1]; the reference's operation order (clamp at
+// run time)
+enum { FK_CLAMP = 256, FK_EXACT = 512 };
 
 struct SweepParams {
   int kind, constr01;
   float dt, anisAlpha;
+  float negZero = -0.0f;  // see mcfExactStrip
 };
 
 // Correctly rounded scalar ops; no contraction, so results follow the written
@@ -144,6 +147,12 @@ struct PlaneJac {
   float r1[6], sy[4];
 };
 
+// MCF in the reference's operation order: the three rows' centre columns, the centre
+// row's outer columns, and the half y-differences of the outer columns.
+struct PlaneMcfX {
+  float r0[4], r1[6], r2[4], h0, h5;
+};
+
 // Reads one plane from the FP32 ring: row0 = row y-1 at column x-1; rows RS apart.
 template <int RS>
 __device__ __forceinline__ void loadPlane(const float *row0, PlaneRaw &P) {
@@ -179,6 +188,17 @@ __device__ __forceinline__ void loadPlane(const float *row0, PlaneJac &P) {
   const float4 v = *reinterpret_cast<const float4 *>(row0 + 2 * RS + 1);
   const float2 s01 = add2(pr(u.x, u.y), pr(v.x, v.y)), s23 = add2(pr(u.z, u.w), pr(v.z, v.w));
   P.sy[0] = s01.x; P.sy[1] = s01.y; P.sy[2] = s23.x; P.sy[3] = s23.y;
+}
+
+template <int RS>
+__device__ __forceinline__ void loadPlane(const float *row0, PlaneMcfX &P) {
+  loadRow1<RS>(row0, P.r1);
+  const float4 u = *reinterpret_cast<const float4 *>(row0 + 1);
+  const float4 v = *reinterpret_cast<const float4 *>(row0 + 2 * RS + 1);
+  P.r0[0] = u.x; P.r0[1] = u.y; P.r0[2] = u.z; P.r0[3] = u.w;
+  P.r2[0] = v.x; P.r2[1] = v.y; P.r2[2] = v.z; P.r2[3] = v.w;
+  P.h0 = __fmul_rn(0.5f, __fsub_rn(row0[2 * RS], row0[0]));
+  P.h5 = __fmul_rn(0.5f, __fsub_rn(row0[2 * RS + 5], row0[5]));
 }
 
 // 1/x from the hardware's approximate reciprocal (PTX rcp.approx.ftz.f32).
@@ -237,6 +257,70 @@ __device__ __forceinline__ void mcfFastStrip(const PlaneMcf &Pm, const PlaneMcf 
     const float D0 = fminf(fmaxf(Hr.x, -0.1f), 0.1f), D1 = fminf(fmaxf(Hr.y, -0.1f), 0.1f);
     out[2 * h] = CLAMP01 ? __saturatef(f0.x + D0) : f0.x + D0;
     out[2 * h + 1] = CLAMP01 ? __saturatef(f0.y + D1) : f0.y + D1;
+  }
+}
+
+// MCF of the strip's four voxels in the reference's operation order: bit for bit
+// mcfExact, two voxels per instruction where the operands pair up (a packed operation
+// rounds each lane as the scalar one does, and a product's operand order does not change
+// it).  Differences that neighbouring voxels share (f_y at x+1 is the next voxel's own
+// f_y) are formed once.  The compiler fuses a packed product into the packed sum that
+// reads it, whatever its rounding modifier says, so a product that feeds a sum is formed
+// as fma(a, b, -0) with the -0 a run-time value: the same rounding, and nothing left to
+// fuse.  Products with 2 are exact, and may be fused.
+__device__ __forceinline__ void mcfExactStrip(const PlaneMcfX &Pm, const PlaneMcfX &P0, const PlaneMcfX &Pp,
+                                              float dt, float negZero, int constr01, float out[4]) {
+  const float2 hh = pr(0.5f, 0.5f), two = pr(2.0f, 2.0f), nz = pr(negZero, negZero);
+  auto mulx = [&](float2 a, float2 b) { return fma2(a, b, nz); };
+  float hy[6], hz[6];  // f_y, f_z at columns x-1 .. x+4
+  hy[0] = P0.h0; hy[5] = P0.h5;
+  hz[0] = __fmul_rn(0.5f, __fsub_rn(Pp.r1[0], Pm.r1[0]));
+  hz[5] = __fmul_rn(0.5f, __fsub_rn(Pp.r1[5], Pm.r1[5]));
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int c = 1 + 2 * h, k = 2 * h;
+    const float2 y = mul2(hh, sub2(pr(P0.r2[k], P0.r2[k + 1]), pr(P0.r0[k], P0.r0[k + 1])));
+    const float2 z = mul2(hh, sub2(pr(Pp.r1[c], Pp.r1[c + 1]), pr(Pm.r1[c], Pm.r1[c + 1])));
+    hy[c] = y.x; hy[c + 1] = y.y; hz[c] = z.x; hz[c + 1] = z.y;
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int c = 1 + 2 * h, k = 2 * h;
+    const float *w = P0.r1;
+    const float2 f0 = pr(w[c], w[c + 1]);
+    const float2 fx = mul2(hh, pr(__fsub_rn(w[c + 1], w[c - 1]), __fsub_rn(w[c + 2], w[c])));
+    const float2 fy = pr(hy[c], hy[c + 1]), fz = pr(hz[c], hz[c + 1]);
+    const float2 f02 = mul2(two, f0);
+    const float2 fxx = sub2(pr(__fadd_rn(w[c - 1], w[c + 1]), __fadd_rn(w[c], w[c + 2])), f02);
+    const float2 fyy = sub2(add2(pr(P0.r0[k], P0.r0[k + 1]), pr(P0.r2[k], P0.r2[k + 1])), f02);
+    const float2 fzz = sub2(add2(pr(Pm.r1[c], Pm.r1[c + 1]), pr(Pp.r1[c], Pp.r1[c + 1])), f02);
+    const float2 fyx = mul2(hh, pr(__fsub_rn(hy[c + 1], hy[c - 1]), __fsub_rn(hy[c + 2], hy[c])));
+    const float2 fzx = mul2(hh, pr(__fsub_rn(hz[c + 1], hz[c - 1]), __fsub_rn(hz[c + 2], hz[c])));
+    const float2 fzu = mulx(hh, sub2(pr(Pp.r2[k], Pp.r2[k + 1]), pr(Pm.r2[k], Pm.r2[k + 1])));
+    const float2 fzd = mulx(hh, sub2(pr(Pp.r0[k], Pp.r0[k + 1]), pr(Pm.r0[k], Pm.r0[k + 1])));
+    const float2 fzy = mul2(hh, sub2(fzu, fzd));
+    const float2 xx = mulx(fx, fx), yy = mulx(fy, fy), zz = mulx(fz, fz);
+    const float2 xy = add2(xx, yy);
+    float2 H = add2(add2(mulx(add2(yy, zz), fxx), mulx(add2(xx, zz), fyy)), mulx(xy, fzz));
+    const float2 cross = add2(add2(mulx(mul2(fx, fy), fyx), mulx(mul2(fx, fz), fzx)), mulx(mul2(fy, fz), fzy));
+    H = sub2(H, mul2(two, cross));
+    const float2 g2 = add2(xy, zz);
+    H.x = g2.x > 1e-7f ? __fdiv_rn(H.x, g2.x) : 0.0f;
+    H.y = g2.y > 1e-7f ? __fdiv_rn(H.y, g2.y) : 0.0f;
+    float2 D = mul2(pr(dt, dt), H);
+    D.x = D.x < -0.1f ? -0.1f : D.x; D.y = D.y < -0.1f ? -0.1f : D.y;
+    D.x = D.x > 0.1f ? 0.1f : D.x; D.y = D.y > 0.1f ? 0.1f : D.y;
+    const float2 v = add2(f0, D);
+    out[k] = v.x; out[k + 1] = v.y;
+  }
+  if (constr01) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      float v = out[i];
+      v = v > 0.0f ? v : 0.0f;
+      v = v < 1.0f ? v : 1.0f;
+      out[i] = v;
+    }
   }
 }
 
