@@ -438,6 +438,9 @@ extern "C" int msbg_gpu_create(msbg_gpu_ctx **out, int sx, int sy, int sz, int b
   ALLOC(ctx->dColorBids, nB * 4);
   ALLOC(ctx->dScanPartial, (size_t)nPart * 8);
   ALLOC(ctx->dCounters, kNumCounters * 8);
+  const auto groups = [](int64_t n) { return (n + 3) / 4; };
+  const int64_t n4 = groups(ctx->nbx) * groups(ctx->nby) * groups(ctx->nbz);
+  ALLOC(ctx->dOccupancy, (size_t)(n4 + groups(groups(ctx->nbx)) * groups(groups(ctx->nby)) * groups(groups(ctx->nbz))));
   ALLOC(ctx->dStatus, 16);
 #undef ALLOC
   if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->hCounters, kNumCounters * 8);
@@ -476,7 +479,7 @@ extern "C" int msbg_gpu_destroy(msbg_gpu_ctx *ctx) {
   cudaFree(ctx->dSlot); cudaFree(ctx->dActive); cudaFree(ctx->dColorBids);
   if (ctx->dListMark) cudaFree(ctx->dListMark);
   if (ctx->dListBids) cudaFree(ctx->dListBids);
-  cudaFree(ctx->dScanPartial); cudaFree(ctx->dCounters); cudaFree(ctx->dStatus);
+  cudaFree(ctx->dScanPartial); cudaFree(ctx->dCounters); cudaFree(ctx->dStatus); cudaFree(ctx->dOccupancy);
   if (ctx->hCounters) cudaFreeHost(ctx->hCounters);
   if (ctx->hSmall) cudaFreeHost(ctx->hSmall);
   for (auto &c : ctx->ch) {

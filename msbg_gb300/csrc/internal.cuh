@@ -88,6 +88,7 @@ struct msbg_gpu_ctx {
   int64_t *dCounters = nullptr;  // [kNumCounters], see kColorTot
   int64_t *hCounters = nullptr;  // pinned mirror
   int64_t *hSmall = nullptr;     // pinned, kSmallReadBytes: target of readSmall
+  uint8_t *dOccupancy = nullptr; // render: value blocks per 4^3 and 16^3 group of blocks
   int *dStatus = nullptr;        // device-side error bits (bounded waits that gave up)
   bool layoutValid = false;
   int64_t nActive = 0;
