@@ -25,6 +25,7 @@
 // table of the 27 blocks around it.
 #include <cuda_bf16.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -34,6 +35,7 @@ namespace msbg {
 
 constexpr int kWnLayers = 4;
 constexpr int kWnCh[kWnLayers + 1] = {2, 16, 16, 16, 2};
+constexpr int kBwdParts = 304;  // persistent CTAs of the weight gradients: two per SM
 
 struct WarmNetState {
   int64_t layoutStamp = -1;
@@ -49,6 +51,7 @@ struct WarmNetState {
   float *t0a = nullptr, *t0b = nullptr;  // level-0 temporaries
   double *dScal = nullptr, *hScal = nullptr;
   double *dPart = nullptr;
+  float *bwdPart = nullptr;        // [kBwdParts] weight and bias sums of one layer
   int nPart = 0;
   int step = 0;
   int lossMode = 0;  // 0 coarse, 1 residual
@@ -667,7 +670,291 @@ __global__ void __launch_bounds__(kTcThreads, BS1 == 16 ? 3 : 2) kConvTcStaged(W
 
 
 // ---------------------------------------------------------------------------------
-// backward convolutions (CUDA cores; FP32)
+// backward convolutions on level-1 blocks of edge 16 and 8 (CUDA cores; FP32)
+// ---------------------------------------------------------------------------------
+// Both gradients are FP32 contractions over 27 taps (their operands are FP32, so the BF16
+// tensor path of the forward pass would lose bits).  The bound is the FP32 pipe: 4.6 GFMA
+// a 16-16 layer on 663 k cells, 115 us at 128 lanes per SM and clock.  The forms below
+// stage a tile of 512 cells with its halo in shared memory once and keep enough products
+// per shared-memory load (11 to 24) for the packed FMAs to be the limit.  Measured on that
+// layout: kBwdData 223 us and kBwdWeight 241 us for a 16-16 layer (52% and 48% of the FP32
+// pipe); a step's three data and four weight launches 495 and 438 us, against 2703 and
+// 2854 us with the neighbours read from global memory per tap (the forms below, kept for
+// blocks of edge 4); the whole loss and gradient 6.02 -> 1.57 ms.
+// Upstream gradients arrive masked by their layer's ReLU: kBwdData masks what it writes.
+template <int BS1>
+struct BwdTile {
+  static constexpr int L = BS1 == 16 ? 4 : 3;
+  static constexpr int TX = BS1, TY = 8, TZ = BS1 == 16 ? 4 : 8;  // 512 cells
+  static constexpr int HX = TX + 2, HY = TY + 2, HZ = TZ + 2, NH = HX * HY * HZ;
+  static constexpr int TPB = BS1 * BS1 * BS1 / 512;  // tiles per block
+};
+
+// Slots of the 27 blocks around a tile's block, and the tile's first cell in it.
+template <int BS1>
+__device__ __forceinline__ void bwdOrigin(const WnGeom &g, int64_t tile, int *nbs, int64_t &s, int &y0, int &z0) {
+  using T = BwdTile<BS1>;
+  s = tile / T::TPB;
+  const int part = (int)(tile % T::TPB);
+  y0 = (part % (BS1 / T::TY)) * T::TY;
+  z0 = (part / (BS1 / T::TY)) * T::TZ;
+  if (threadIdx.x < 27) nbs[threadIdx.x] = g.nbr27[s * 27 + threadIdx.x];
+}
+// index of the level-1 cell at halo position (hx, hy, hz) of the tile, or -1
+template <int BS1>
+__device__ __forceinline__ int64_t bwdCell(const int *nbs, int y0, int z0, int hx, int hy, int hz) {
+  using T = BwdTile<BS1>;
+  const int x = hx - 1, y = y0 + hy - 1, z = z0 + hz - 1, m = BS1 - 1;
+  const int s = nbs[(x >> T::L) + 1 + 3 * ((y >> T::L) + 1) + 9 * ((z >> T::L) + 1)];
+  if (s < 0) return -1;
+  return ((int64_t)s << (3 * T::L)) + ((((z & m) << T::L) + (y & m)) << T::L) + (x & m);
+}
+
+// gx[c][i] = sum_tap sum_o W[tap][i][o] gp[c - tap][o], masked by below[c][i] > 0.
+// A thread takes 4 cells along z and 8 input channels: per (ey, ex) column and 4 upstream
+// channels it loads 6 cells once for the three z taps and 24 weights that the warp shares,
+// for 384 products in pairs over o (the two halves of a pair are added at the end).  Lanes
+// run along x, so the 16-byte loads of a plane [channel quad][z][y][x] do not conflict.
+template <int BS1, int COUT>
+constexpr size_t bwdDataSmem() { return ((size_t)BwdTile<BS1>::NH + 27 * 16) * COUT * 4; }
+template <int BS1, int COUT>
+__global__ void __launch_bounds__(256, 2) kBwdData(WnGeom g, const float *__restrict__ gp, const float *__restrict__ below,
+                                                   const __nv_bfloat16 *__restrict__ w, float *__restrict__ gx) {
+  using T = BwdTile<BS1>;
+  constexpr int V = COUT < 4 ? 2 : 4, NQ = COUT / V;  // channels per load, loads per cell
+  using VT = std::conditional_t<V == 4, float4, float2>;
+  extern __shared__ __align__(16) unsigned char bwdSmem[];
+  VT *sg = reinterpret_cast<VT *>(bwdSmem);   // [NQ][HZ][HY][HX]
+  VT *sw = sg + NQ * T::NH;                   // [27][NQ][16]: V consecutive o of an input channel
+  __shared__ int nbs[27];
+  const int tid = threadIdx.x;
+  int64_t s;
+  int y0, z0;
+  bwdOrigin<BS1>(g, blockIdx.x, nbs, s, y0, z0);
+  for (int k = tid; k < 27 * NQ * 16; k += 256) {
+    const int i = k % 16, q = (k / 16) % NQ, t = k / (16 * NQ);
+    float v[V];
+#pragma unroll
+    for (int o = 0; o < V; o++) v[o] = __bfloat162float(w[(t * 16 + i) * COUT + q * V + o]);
+    if constexpr (V == 4) sw[k] = make_float4(v[0], v[1], v[2], v[3]);
+    else sw[k] = make_float2(v[0], v[1]);
+  }
+  __syncthreads();
+  for (int k = tid; k < NQ * T::NH; k += 256) {
+    const int q = k % NQ, h = k / NQ;  // a cell's channels are contiguous in memory
+    const int64_t c = bwdCell<BS1>(nbs, y0, z0, h % T::HX, (h / T::HX) % T::HY, h / (T::HX * T::HY));
+    VT v;
+    if constexpr (V == 4) v = make_float4(0.f, 0.f, 0.f, 0.f);
+    else v = make_float2(0.f, 0.f);
+    if (c >= 0) v = reinterpret_cast<const VT *>(gp)[c * NQ + q];
+    sg[q * T::NH + h] = v;
+  }
+  __syncthreads();
+  const int lane = tid & 31, warp = tid >> 5, ih = lane >> 4;
+  const int x = lane & (BS1 - 1);
+  const int y = BS1 == 16 ? warp : ((lane >> 3) & 1) + 2 * (warp & 3);
+  const int zc = BS1 == 16 ? 0 : 4 * (warp >> 2);
+  float2 acc[4][8];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[k][i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int col = 0; col < 9; col++) {
+    const int ex = col % 3 - 1, ey = col / 3 - 1;
+    const int tap = (1 - ex) + 3 * (1 - ey) + 9;  // the tap with ez = 0; ez moves it by -9 ez
+#pragma unroll 1
+    for (int q = 0; q < NQ; q++) {
+      const VT *src = sg + q * T::NH + (zc * T::HY + y + 1 + ey) * T::HX + x + 1 + ex;
+      VT win[6];
+#pragma unroll
+      for (int k = 0; k < 6; k++) win[k] = src[k * T::HY * T::HX];
+#pragma unroll
+      for (int ez = -1; ez <= 1; ez++) {
+        const VT *wt = sw + ((tap - 9 * ez) * NQ + q) * 16 + 8 * ih;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const VT wv = wt[i];
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const VT gv = win[k + 1 + ez];
+            acc[k][i] = __ffma2_rn(make_float2(wv.x, wv.y), make_float2(gv.x, gv.y), acc[k][i]);
+            if constexpr (V == 4)
+              acc[k][i] = __ffma2_rn(make_float2(wv.z, wv.w), make_float2(gv.z, gv.w), acc[k][i]);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int64_t c = (s << (3 * T::L)) + ((((z0 + zc + k) << T::L) + y0 + y) << T::L) + x;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int64_t at = c * 4 + 2 * ih + h;
+      const float4 b = reinterpret_cast<const float4 *>(below)[at];
+      const float2 *a = &acc[k][4 * h];
+      reinterpret_cast<float4 *>(gx)[at] =
+          make_float4(b.x > 0.f ? a[0].x + a[0].y : 0.f, b.y > 0.f ? a[1].x + a[1].y : 0.f,
+                      b.z > 0.f ? a[2].x + a[2].y : 0.f, b.w > 0.f ? a[3].x + a[3].y : 0.f);
+    }
+  }
+}
+
+// part[cta][tap][i][o] = sum over the CTA's cells of x[c + tap][i] gp[c][o], and behind them
+// sum gp[c][o].  Nine warps, one per (dy, dz); a lane takes up to 4 input by 4 upstream
+// channels and marches along rows in x with the three x taps' cells in registers, so a cell
+// costs two 16-byte loads for 48 products; lanes left over share the rows.  Row strides are
+// odd multiples of a cell's bytes, so rows next to each other use different banks.  CTAs
+// are persistent, their sums are added in FP64 in a fixed order (kSumBwdParts).
+template <int BS1, int CIN, int COUT>
+struct BwdWeight {
+  using T = BwdTile<BS1>;
+  static constexpr int XS = T::HX + 1, GS = T::TX + 1;  // row strides in cells
+  static constexpr int IV = CIN < 4 ? CIN : 4, OV = COUT < 4 ? COUT : 4;
+  static constexpr int NI = CIN / IV, NO = COUT / OV, PARTS = 32 / (NI * NO);
+  static constexpr int NOUT = 27 * CIN * COUT + COUT;
+  static constexpr int XF = T::HZ * T::HY * XS * CIN, GF = T::TZ * T::TY * GS * COUT;
+  static constexpr size_t smem = (size_t)(XF + GF) * 4;
+};
+constexpr int kBwdWThreads = 288;
+template <int N> struct VecN;
+template <> struct VecN<2> { using V = float2; };
+template <> struct VecN<4> { using V = float4; };
+
+template <int BS1, int CIN, int COUT, bool NORM>
+__global__ void __launch_bounds__(kBwdWThreads, 2) kBwdWeight(WnGeom g, const float *__restrict__ x,
+                                                              const float *__restrict__ gp,
+                                                              const double *__restrict__ sc, int64_t nTiles,
+                                                              float *__restrict__ part) {
+  using T = BwdTile<BS1>;
+  using W = BwdWeight<BS1, CIN, COUT>;
+  constexpr int IV = W::IV, OV = W::OV;
+  using XV = typename VecN<IV>::V;
+  using GV = typename VecN<OV>::V;
+  extern __shared__ __align__(16) unsigned char bwdSmem[];
+  float *sx = reinterpret_cast<float *>(bwdSmem), *sg = sx + W::XF;
+  __shared__ int nbs[27];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int dy = warp % 3, dz = warp / 3;  // 0..2: the tap's offset + 1
+  const int oq = lane % W::NO, iq = (lane / W::NO) % W::NI, rp = lane / (W::NO * W::NI);
+  const float s0 = NORM ? (float)sc[1] : 1.f, s1 = NORM ? (float)sc[2] : 1.f;
+  float2 acc[3][IV][OV / 2];
+  float gsum[OV];
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int i = 0; i < IV; i++)
+#pragma unroll
+      for (int o = 0; o < OV / 2; o++) acc[d][i][o] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int o = 0; o < OV; o++) gsum[o] = 0.f;
+  for (int64_t tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
+    int64_t s;
+    int y0, z0;
+    __syncthreads();  // the previous tile is read
+    bwdOrigin<BS1>(g, tile, nbs, s, y0, z0);
+    __syncthreads();
+    for (int k = tid; k < T::NH * W::NI; k += kBwdWThreads) {
+      const int q = k % W::NI, h = k / W::NI, hx = h % T::HX, hy = (h / T::HX) % T::HY, hz = h / (T::HX * T::HY);
+      const int64_t c = bwdCell<BS1>(nbs, y0, z0, hx, hy, hz);
+      XV v;
+      if constexpr (IV == 4) v = make_float4(0.f, 0.f, 0.f, 0.f);
+      else v = make_float2(0.f, 0.f);
+      if (c >= 0) {
+        v = reinterpret_cast<const XV *>(x)[c * W::NI + q];
+        if constexpr (NORM) { v.x *= s0; v.y = v.y * s1 - 1.0f; }
+      }
+      reinterpret_cast<XV *>(sx)[((hz * T::HY + hy) * W::XS + hx) * W::NI + q] = v;
+    }
+    for (int k = tid; k < 512 * W::NO; k += kBwdWThreads) {
+      const int q = k % W::NO, c = k / W::NO, cx = c % T::TX, cy = (c / T::TX) % T::TY, cz = c / (T::TX * T::TY);
+      const int64_t at = (s << (3 * T::L)) + ((((z0 + cz) << T::L) + y0 + cy) << T::L) + cx;
+      reinterpret_cast<GV *>(sg)[((cz * T::TY + cy) * W::GS + cx) * W::NO + q] =
+          reinterpret_cast<const GV *>(gp)[at * W::NO + q];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int r = rp; r < T::TY * T::TZ; r += W::PARTS) {
+      const int ry = r % T::TY, rz = r / T::TY;
+      const XV *xr = reinterpret_cast<const XV *>(sx) + ((rz + dz) * T::HY + ry + dy) * W::XS * W::NI + iq;
+      const GV *gr = reinterpret_cast<const GV *>(sg) + (rz * T::TY + ry) * W::GS * W::NO + oq;
+      XV win[3];
+      win[0] = xr[0];
+      win[1] = xr[W::NI];
+#pragma unroll
+      for (int c = 0; c < T::TX; c++) {
+        win[(c + 2) % 3] = xr[(c + 2) * W::NI];
+        const GV gv = gr[c * W::NO];
+        float gs[OV];
+        if constexpr (OV == 4) { gs[0] = gv.x; gs[1] = gv.y; gs[2] = gv.z; gs[3] = gv.w; }
+        else { gs[0] = gv.x; gs[1] = gv.y; }
+        if (warp == 4) {
+#pragma unroll
+          for (int o = 0; o < OV; o++) gsum[o] += gs[o];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const XV xv = win[(c + d) % 3];
+          float xs[IV];
+          if constexpr (IV == 4) { xs[0] = xv.x; xs[1] = xv.y; xs[2] = xv.z; xs[3] = xv.w; }
+          else { xs[0] = xv.x; xs[1] = xv.y; }
+#pragma unroll
+          for (int i = 0; i < IV; i++)
+#pragma unroll
+            for (int o = 0; o < OV / 2; o++)
+              acc[d][i][o] = __ffma2_rn(make_float2(xs[i], xs[i]), make_float2(gs[2 * o], gs[2 * o + 1]), acc[d][i][o]);
+        }
+      }
+    }
+  }
+  float *dst = part + (int64_t)blockIdx.x * W::NOUT;
+  auto lanesSum = [&](float v) {  // over the lanes that share a channel pair (the row parts)
+#pragma unroll
+    for (int o = W::NI * W::NO; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int i = 0; i < IV; i++)
+#pragma unroll
+      for (int o = 0; o < OV / 2; o++) {
+        const float a = lanesSum(acc[d][i][o].x), b = lanesSum(acc[d][i][o].y);
+        if (rp == 0) {
+          float *q = dst + ((d + 3 * dy + 9 * dz) * CIN + iq * IV + i) * COUT + oq * OV + 2 * o;
+          q[0] = a;
+          q[1] = b;
+        }
+      }
+  if (warp == 4) {
+#pragma unroll
+    for (int o = 0; o < OV; o++) {
+      const float v = lanesSum(gsum[o]);
+      if (rp == 0 && iq == 0) dst[27 * CIN * COUT + oq * OV + o] = v;
+    }
+  }
+}
+
+// gw, gb: the CTAs' sums added in FP64; 32 outputs a CTA, 8 threads an output
+__global__ void __launch_bounds__(256) kSumBwdParts(const float *__restrict__ part, int nParts, int nOut, int nW,
+                                                    float *__restrict__ gw, float *__restrict__ gb) {
+  __shared__ double sum[8][32];
+  const int o = blockIdx.x * 32 + (threadIdx.x & 31), k = threadIdx.x >> 5;
+  double a = 0.0;
+  if (o < nOut)
+    for (int p = k; p < nParts; p += 8) a += (double)part[(int64_t)p * nOut + o];
+  sum[k][threadIdx.x & 31] = a;
+  __syncthreads();
+  if (k == 0 && o < nOut) {
+#pragma unroll
+    for (int j = 1; j < 8; j++) a += sum[j][threadIdx.x];
+    if (o < nW) gw[o] = (float)a; else gb[o - nW] = (float)a;
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// backward convolutions on smaller blocks (CUDA cores; FP32)
 // ---------------------------------------------------------------------------------
 // gx[c][i] = sum_tap sum_o W[tap][i][o] * gpre[c - tap][o], gpre = gy * (y > 0) when
 // the layer has a ReLU.  Written for the layers above the input only.
@@ -805,7 +1092,7 @@ namespace msbg {
 
 void warmNetFree(WarmNetState *w) {
   if (!w) return;
-  void *ptrs[] = {w->nbr27, w->x1, w->gx1, w->t0a, w->t0b, w->dScal, w->dPart, w->gact[0], w->gact[1]};
+  void *ptrs[] = {w->nbr27, w->x1, w->gx1, w->t0a, w->t0b, w->dScal, w->dPart, w->bwdPart, w->gact[0], w->gact[1]};
   for (void *p : ptrs) if (p) cudaFree(p);
   for (int l = 0; l < kWnLayers; l++) {
     void *q[] = {w->w32[l], w->bias[l], w->wq[l], w->gw[l], w->gb[l], w->mw[l], w->vw[l], w->mb[l], w->vb[l]};
@@ -859,6 +1146,7 @@ static int wnEnsure(msbg_gpu_ctx *ctx) {
     MSBG_CUDA(ctx, cudaMallocHost((void **)&w->hScal, 16 * 8));
     w->nPart = 152 * 8;
     MSBG_CUDA(ctx, cudaMalloc(&w->dPart, (size_t)w->nPart * 2 * 8));
+    MSBG_CUDA(ctx, cudaMalloc(&w->bwdPart, (size_t)kBwdParts * (27 * 16 * 16 + 16) * 4));
   }
   WarmNetState *w = ctx->warmnet;
   if (w->layoutStamp == ctx->layoutStamp) return MSBG_GPU_OK;
@@ -950,7 +1238,77 @@ static int wnForward(msbg_gpu_ctx *ctx, const float *b0, float *x0) {
   return MSBG_GPU_OK;
 }
 
-// loss into hScal[4] (and dScal[4]); gradients into gw/gb (zeroed first)
+// one layer's weight and bias gradients, tiled form
+template <int BS1, int CIN, int COUT, bool NORM>
+static int wnBwdWeight(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g, int l, const float *gp) {
+  using W = BwdWeight<BS1, CIN, COUT>;
+  static bool attr = false;
+  if (!attr) {
+    MSBG_CUDA(ctx, cudaFuncSetAttribute(kBwdWeight<BS1, CIN, COUT, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)W::smem));
+    attr = true;
+  }
+  const int64_t nTiles = w->n1 / 512;
+  const int grid = (int)(nTiles < kBwdParts ? nTiles : kBwdParts);
+  MSBG_LAUNCH(ctx, (kBwdWeight<BS1, CIN, COUT, NORM>), (unsigned)grid, kBwdWThreads, W::smem, g, w->act[l], gp, w->dScal,
+              nTiles, w->bwdPart);
+  MSBG_LAUNCH(ctx, kSumBwdParts, (unsigned)((W::NOUT + 31) / 32), 256, 0, w->bwdPart, grid, W::NOUT, wnWeights(l),
+              w->gw[l], w->gb[l]);
+  return MSBG_GPU_OK;
+}
+// the gradient of a layer's input, masked by the ReLU below it
+template <int BS1, int COUT>
+static int wnBwdData(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g, int l, const float *gp, float *gx) {
+  constexpr size_t smem = bwdDataSmem<BS1, COUT>();
+  static bool attr = false;
+  if (!attr) {
+    MSBG_CUDA(ctx, cudaFuncSetAttribute(kBwdData<BS1, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr = true;
+  }
+  MSBG_LAUNCH(ctx, (kBwdData<BS1, COUT>), (unsigned)(w->n1 / 512), 256, smem, g, gp, w->act[l], w->wq[l], gx);
+  return MSBG_GPU_OK;
+}
+template <int BS1>
+static int wnBackwardTiles(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g) {
+  int rc;
+  if ((rc = wnBwdWeight<BS1, 16, 2, false>(ctx, w, g, 3, w->gact[0]))) return rc;
+  if ((rc = wnBwdData<BS1, 2>(ctx, w, g, 3, w->gact[0], w->gact[1]))) return rc;
+  if ((rc = wnBwdWeight<BS1, 16, 16, false>(ctx, w, g, 2, w->gact[1]))) return rc;
+  if ((rc = wnBwdData<BS1, 16>(ctx, w, g, 2, w->gact[1], w->gact[0]))) return rc;
+  if ((rc = wnBwdWeight<BS1, 16, 16, false>(ctx, w, g, 1, w->gact[0]))) return rc;
+  if ((rc = wnBwdData<BS1, 16>(ctx, w, g, 1, w->gact[0], w->gact[1]))) return rc;
+  return wnBwdWeight<BS1, 2, 16, true>(ctx, w, g, 0, w->gact[1]);
+}
+
+// all gradients from the upstream gradient of the output in gact[0] [n1][2]
+static int wnBackward(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g) {
+  if (w->n1 > 0 && g.bs == 16) return wnBackwardTiles<16>(ctx, w, g);
+  if (w->n1 > 0 && g.bs == 8) return wnBackwardTiles<8>(ctx, w, g);
+  for (int l = 0; l < kWnLayers; l++) {
+    MSBG_CUDA(ctx, cudaMemsetAsync(w->gw[l], 0, wnWeights(l) * 4, ctx->stream));
+    MSBG_CUDA(ctx, cudaMemsetAsync(w->gb[l], 0, kWnCh[l + 1] * 4, ctx->stream));
+  }
+  const unsigned gr = wnGrid(w->n1);
+  const unsigned gwc = (unsigned)((w->n1 + kWChunk - 1) / kWChunk);
+  // layer 3 (no ReLU): upstream gact[0] [n1][2]
+  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 2, false, false>), gwc, 256, 0, g, w->act[3], w->gact[0], w->act[4], w->dScal,
+              w->gw[3], w->gb[3]);
+  MSBG_LAUNCH(ctx, (kConvBwdData<16, 2, false>), gr, 256, 0, g, w->gact[0], w->act[4], w->wq[3], w->gact[1]);
+  // layer 2: upstream gact[1] [n1][16], ReLU on act[3]
+  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 16, true, false>), gwc, 256, 0, g, w->act[2], w->gact[1], w->act[3],
+              w->dScal, w->gw[2], w->gb[2]);
+  MSBG_LAUNCH(ctx, (kConvBwdData<16, 16, true>), gr, 256, 0, g, w->gact[1], w->act[3], w->wq[2], w->gact[0]);
+  // layer 1
+  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 16, true, false>), gwc, 256, 0, g, w->act[1], w->gact[0], w->act[2],
+              w->dScal, w->gw[1], w->gb[1]);
+  MSBG_LAUNCH(ctx, (kConvBwdData<16, 16, true>), gr, 256, 0, g, w->gact[0], w->act[2], w->wq[1], w->gact[1]);
+  // layer 0 (input scaling applied on load)
+  MSBG_LAUNCH(ctx, (kConvBwdWeight<2, 16, true, true>), gwc, 256, 0, g, w->act[0], w->gact[1], w->act[1], w->dScal,
+              w->gw[0], w->gb[0]);
+  return MSBG_GPU_OK;
+}
+
+// loss into hScal[4] (and dScal[4]); gradients into gw/gb
 static int wnLossGrad(msbg_gpu_ctx *ctx, const float *b0, const float *xs0) {
   PoissonState *ps = ctx->poisson;
   WarmNetState *w = ctx->warmnet;
@@ -975,27 +1333,7 @@ static int wnLossGrad(msbg_gpu_ctx *ctx, const float *b0, const float *xs0) {
   MSBG_LAUNCH(ctx, kScaleInPlace, wnGrid(n0), 256, 0, w->t0a, w->dScal + 4, w->dScal + 5, 2.0f, n0);  // g0
   MSBG_LAUNCH(ctx, kWnHeadBack, gridFor(w->n2, 256), 256, 0, w->t0a, w->dScal, g.L, w->n2, (float2 *)w->gact[0]);
   }
-  for (int l = 0; l < kWnLayers; l++) {
-    MSBG_CUDA(ctx, cudaMemsetAsync(w->gw[l], 0, wnWeights(l) * 4, ctx->stream));
-    MSBG_CUDA(ctx, cudaMemsetAsync(w->gb[l], 0, kWnCh[l + 1] * 4, ctx->stream));
-  }
-  const unsigned gr = wnGrid(w->n1);
-  const unsigned gwc = (unsigned)((w->n1 + kWChunk - 1) / kWChunk);
-  // layer 3 (no ReLU): upstream gact[0] [n1][2]
-  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 2, false, false>), gwc, 256, 0, g, w->act[3], w->gact[0], w->act[4], w->dScal,
-              w->gw[3], w->gb[3]);
-  MSBG_LAUNCH(ctx, (kConvBwdData<16, 2, false>), gr, 256, 0, g, w->gact[0], w->act[4], w->wq[3], w->gact[1]);
-  // layer 2: upstream gact[1] [n1][16], ReLU on act[3]
-  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 16, true, false>), gwc, 256, 0, g, w->act[2], w->gact[1], w->act[3],
-              w->dScal, w->gw[2], w->gb[2]);
-  MSBG_LAUNCH(ctx, (kConvBwdData<16, 16, true>), gr, 256, 0, g, w->gact[1], w->act[3], w->wq[2], w->gact[0]);
-  // layer 1
-  MSBG_LAUNCH(ctx, (kConvBwdWeight<16, 16, true, false>), gwc, 256, 0, g, w->act[1], w->gact[0], w->act[2],
-              w->dScal, w->gw[1], w->gb[1]);
-  MSBG_LAUNCH(ctx, (kConvBwdData<16, 16, true>), gr, 256, 0, g, w->gact[0], w->act[2], w->wq[1], w->gact[1]);
-  // layer 0 (input scaling applied on load)
-  MSBG_LAUNCH(ctx, (kConvBwdWeight<2, 16, true, true>), gwc, 256, 0, g, w->act[0], w->gact[1], w->act[1], w->dScal,
-              w->gw[0], w->gb[0]);
+  if ((rc = wnBackward(ctx, w, g))) return rc;
   MSBG_CUDA(ctx, cudaMemcpyAsync(w->hScal + 4, w->dScal + 4, 2 * 8, cudaMemcpyDeviceToHost, ctx->stream));
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return MSBG_GPU_OK;
