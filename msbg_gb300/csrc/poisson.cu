@@ -426,6 +426,7 @@ static int allocT(msbg_gpu_ctx *ctx, T **p, int64_t n) {
 void poissonFree(PoissonState *ps) {
   if (!ps) return;
   for (auto &L : ps->levels) {
+    for (void *q : {(void *)L.nbr, (void *)L.parent, (void *)L.child, (void *)L.bpar}) if (q) cudaFree(q);
     if (L.ownsIndex) {
       if (L.slot) cudaFree(L.slot);
       if (L.active) cudaFree(L.active);
@@ -437,6 +438,7 @@ void poissonFree(PoissonState *ps) {
     for (void *q : {P->vr, P->vp, P->vz, P->vs, P->ve, P->vb}) if (q) cudaFree(q);
   }
   if (ps->dCoarseInv) cudaFree(ps->dCoarseInv);
+  if (ps->dTailBar) cudaFree(ps->dTailBar);
   if (ps->dNbr) cudaFree(ps->dNbr);
   if (ps->dBpar) cudaFree(ps->dBpar);
   if (ps->dParList) cudaFree(ps->dParList);
@@ -513,7 +515,8 @@ static int buildHierarchy(msbg_gpu_ctx *ctx, PoissonState *ps) {
   MSBG_CUDA(ctx, cudaMalloc(&ps->dPartial, (size_t)ps->nPartial * 2 * sizeof(double)));
   MSBG_CUDA(ctx, cudaMalloc(&ps->dScal, 32 * sizeof(double)));
   MSBG_CUDA(ctx, cudaMallocHost((void **)&ps->hScal, 32 * sizeof(double)));
-  return blkBuildTables(ctx, ps);
+  if ((rc = blkBuildTables(ctx, ps))) return rc;
+  return tailBuildTables(ctx, ps);
 }
 
 // Inverse of a symmetric positive definite matrix (row-major, n x n) through its
@@ -714,6 +717,10 @@ static int vcycleT(msbg_gpu_ctx *ctx, PoissonState *ps, const PrecSet &P, size_t
     }
     return MSBG_GPU_OK;
   }
+  if (l > 0 && x == a.x() && b == a.b()) {  // the small levels in one launch
+    bool done = false;
+    if ((rc = coarseTail<V>(ctx, ps, P, l, &done)) || done) return rc;
+  }
   if ((rc = smoothLevel<V>(ctx, ps, P, l, x, b, ps->preSweeps, false, kFirstZero, nullptr))) return rc;
   const MgLevel &C = ps->levels[l + 1];
   const Arr<V> ac{P, l + 1};
@@ -803,6 +810,8 @@ static int checkStatus(msbg_gpu_ctx *ctx) {
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st) {
     MSBG_CUDA(ctx, cudaMemsetAsync(ctx->dStatus, 0, sizeof(int), ctx->stream));
+    if (ctx->poisson && ctx->poisson->dTailBar)
+      MSBG_CUDA(ctx, cudaMemsetAsync(ctx->poisson->dTailBar, 0, 2 * sizeof(unsigned), ctx->stream));
     return fail(ctx, MSBG_GPU_ERR_TIMEOUT, "a bounded device wait timed out (status bits %d)", st);
   }
   return MSBG_GPU_OK;

@@ -166,6 +166,8 @@ struct MgLevel {  // geometry of one level (arrays live in PrecSet)
   int32_t *slot = nullptr, *active = nullptr;
   bool ownsIndex = false;
   bool sameSet = false;  // shares level 0's block set (block edge halved)
+  int32_t *nbr = nullptr, *parent = nullptr, *child = nullptr;  // aggregated levels (poisson_tail.cu); parent: also
+  uint8_t *bpar = nullptr;                                      // the level above the first of them
   int tile = 0;          // tile smoother for this block edge (32, 16, 8), 0 = pointwise red-black
 };
 
@@ -194,6 +196,7 @@ struct PoissonState {
   uint8_t *dBpar = nullptr;
   std::map<std::tuple<const void *, int, int>, CUtensorMap> tmaMaps;  // smoother tensor maps
   int64_t nEven = 0;
+  unsigned *dTailBar = nullptr;  // barrier of the small levels' kernel (poisson_tail.cu)
   int32_t *dListBuf = nullptr;   // block-list calls: slots, parity lists, counters
   double *dListPart = nullptr;   // per-listed-block partial sums
   int64_t listCap = 0;
@@ -236,6 +239,14 @@ BlkGeom blkOf(const PoissonState *ps, const MgLevel &L);
 // Block-structured kernels (poisson_blk.cu), levels with sameSet and bs >= 4.
 // Neighbour table and parity list of the level-0 block set.
 int blkBuildTables(msbg_gpu_ctx *ctx, PoissonState *ps);
+// Face-neighbour table [nAct][6] and coordinate parities of a level's blocks.
+int blkNbrTable(msbg_gpu_ctx *ctx, const MgLevel &L, int32_t *nbr, uint8_t *bpar);
+// The levels below the tile-smoothed ones in one launch (poisson_tail.cu): tables at
+// hierarchy build, then per V-cycle; done: whether it took the levels from l.
+constexpr int64_t kTailMaxCells = 1 << 20;
+int tailBuildTables(msbg_gpu_ctx *ctx, PoissonState *ps);
+template <typename V>
+int coarseTail(msbg_gpu_ctx *ctx, PoissonState *ps, const PrecSet &P, size_t l, bool *done);
 // mode 0: y = A x (dotOut != null: partial sums of x.y to ps->dPartial, summed
 // into *dotOut); mode 1: r = b - A x written to y, or, when bc != null,
 // restricted (sum of 8 children) into the coarse b and the coarse x zeroed;

@@ -737,7 +737,7 @@ __global__ void kNbrTable(const int32_t *__restrict__ active, int64_t nAct, int 
     if (x >= 0 && y >= 0 && z >= 0 && x < nbx && y < nby && z < nbz) v = slot[((int64_t)z * nby + y) * nbx + x];
     nbr[s * 6 + k] = v;
   }
-  even[s] = ((bx + by + bz) & 1) == 0;
+  if (even) even[s] = ((bx + by + bz) & 1) == 0;
   bpar[s] = (uint8_t)((bx & 1) | ((by & 1) << 1) | ((bz & 1) << 2));
 }
 __global__ void kParityList(const int32_t *__restrict__ even, const int64_t *__restrict__ off, int64_t nAct,
@@ -768,6 +768,13 @@ int blkBuildTables(msbg_gpu_ctx *ctx, PoissonState *ps) {
   MSBG_CUDA(ctx, cudaMemcpyAsync(&ne, ctx->dCounters + 6, 8, cudaMemcpyDeviceToHost, ctx->stream));
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ps->nEven = ne;
+  return MSBG_GPU_OK;
+}
+
+int blkNbrTable(msbg_gpu_ctx *ctx, const MgLevel &L, int32_t *nbr, uint8_t *bpar) {
+  if (L.nAct > 0)
+    MSBG_LAUNCH(ctx, kNbrTable, gridFor(L.nAct, 256), 256, 0, L.active, L.nAct, L.nbx, L.nby, L.nbz, L.slot, nbr,
+                (int32_t *)nullptr, bpar);
   return MSBG_GPU_OK;
 }
 
