@@ -14,6 +14,8 @@
 // FP32 staging slab and the finalize quantizes the minimum to the storage type
 // first: rounding is monotonic, so quantize(min) == min(quantize) and the result
 // equals the demo's min over quantized values (src/msbg_demo.cpp:624-628).
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace msbg {
@@ -59,6 +61,7 @@ struct SplatGeom {
   int sx, sy, sz, nbx, nby, log2bs;
   float domMin[3], domMax[3];
   float rScan, distSqMax, distSqMaxInv;
+  float negZero = -0.0f;  // see splatEntries
 };
 
 // A particle's splat box (src/msbg_demo.cpp:571-592): voxels [i1, i2] per axis,
@@ -80,91 +83,165 @@ __device__ __forceinline__ bool splatBox(const SplatGeom &g, float px, float py,
   return b.ix2 >= b.ix1 && b.iy2 >= b.iy1 && b.iz2 >= b.iz1;
 }
 
-// Pass 1, one thread per particle.  Valid particles (the marking loop's domain
-// tests, src/msbg_demo.cpp:358-360, and an owning value block: the demo walks the
-// particle lists of value blocks only, src/msbg_demo.cpp:541-566) get their abort
-// index: the scan position (z, y, x order over the box) of the first in-sphere
-// voxel whose block is not a value block (src/msbg_demo.cpp:613-618), or the box
-// size.  Voxels from that position on are not written.  Every value block the box
-// touches (at most two per axis) counts the particle once.  abortAt = 0 marks a
-// particle that writes nothing.
-__global__ void __launch_bounds__(256) kSplatCount(const float *__restrict__ pts, int64_t n, SplatGeom g,
-                                                   const int32_t *__restrict__ slot, int32_t *__restrict__ abortAt,
-                                                   int32_t *__restrict__ cnt,
-                                                   unsigned long long *__restrict__ nAborted) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float px = pts[3 * i], py = pts[3 * i + 1], pz = pts[3 * i + 2];
-  abortAt[i] = 0;
-  if (px < g.domMin[0] || px > g.domMax[0] || py < g.domMin[1] || py > g.domMax[1] ||
-      pz < g.domMin[2] || pz > g.domMax[2])
-    return;
+// The lists' counters are shared by the particles near each other: a surface's particles
+// come one after another, so thousands of atomics at a time met on the same few hundred
+// addresses (2.05 M particles of the 512^3 workload: 346 us to count, 357 us to scatter).
+// A CTA therefore sums its particles' blocks in a hash table in shared memory and goes to
+// the global counters once per block (@LISTS@).  A block that finds no place within
+// kHashProbes goes to the global counter directly; whether it has a place is the same for
+// every thread and both passes over the particles, since places are never given back.
+constexpr int kListThreads = 512, kHashSize = 2048, kHashProbes = 16;
+struct BlockHash {
+  int key[kHashSize], val[kHashSize];
+};
+__device__ __forceinline__ void hashClear(BlockHash &h) {
+  for (int i = threadIdx.x; i < kHashSize; i += kListThreads) { h.key[i] = -1; h.val[i] = 0; }
+}
+// place of slot sl, claimed if INSERT; -1: none
+template <bool INSERT>
+__device__ __forceinline__ int hashPlace(BlockHash &h, int sl) {
+  unsigned p = ((unsigned)sl * 2654435761u) >> 21;
+  static_assert(kHashSize == 2048, "11 hash bits");
+  for (int k = 0; k < kHashProbes; k++, p = (p + 1) & (kHashSize - 1)) {
+    int at = *(volatile int *)&h.key[p];
+    if (INSERT && at == -1) {
+      at = atomicCAS(&h.key[p], -1, sl);
+      if (at == -1) return (int)p;
+    }
+    if (at == sl) return (int)p;
+    if (!INSERT && at == -1) return -1;
+  }
+  return -1;
+}
+
+// The slots of the value blocks a box touches (at most two per axis), each once, -1 elsewhere.
+__device__ __forceinline__ bool boxSlots(const SplatGeom &g, const SplatBox &b, const int32_t *__restrict__ slot,
+                                         int32_t sl[8]) {
   const int s = g.log2bs;
   const int64_t nxy = (int64_t)g.nbx * g.nby;
-  {
-    const int ix = (int)px, iy = (int)py, iz = (int)pz;
-    if (ix < 0 || ix >= g.sx || iy < 0 || iy >= g.sy || iz < 0 || iz >= g.sz) return;
-    if (slot[(int64_t)(iz >> s) * nxy + (int64_t)(iy >> s) * g.nbx + (ix >> s)] < 0) return;
-  }
-  SplatBox b;
-  if (!splatBox(g, px, py, pz, b)) return;
-  const int nx = b.ix2 - b.ix1 + 1, ny = b.iy2 - b.iy1 + 1, nz = b.iz2 - b.iz1 + 1;
-  const int total = nx * ny * nz;
   const int bx[2] = {b.ix1 >> s, b.ix2 >> s}, by[2] = {b.iy1 >> s, b.iy2 >> s}, bz[2] = {b.iz1 >> s, b.iz2 >> s};
-  int32_t sl[8];
   bool allValue = true;
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    sl[k] = slot[(int64_t)bz[k >> 2] * nxy + (int64_t)by[(k >> 1) & 1] * g.nbx + bx[k & 1]];
-    allValue = allValue && sl[k] >= 0;
+    const bool dup = ((k & 1) && bx[1] == bx[0]) || ((k & 2) && by[1] == by[0]) || ((k & 4) && bz[1] == bz[0]);
+    sl[k] = -1;
+    if (!dup) {
+      sl[k] = slot[(int64_t)bz[k >> 2] * nxy + (int64_t)by[(k >> 1) & 1] * g.nbx + bx[k & 1]];
+      allValue = allValue && sl[k] >= 0;
+    }
   }
-  int abortIdx = total;
-  if (!allValue) {
-    for (int t = 0; t < total; t++) {
-      const int lx = t % nx, rest = t / nx, ly = rest % ny, lz = rest / ny;
-      const int ix = b.ix1 + lx, iy = b.iy1 + ly, iz = b.iz1 + lz;
-      const float dz = __fsub_rn((float)iz, b.z0), dy = __fsub_rn((float)iy, b.y0), dx = __fsub_rn((float)ix, b.x0);
-      const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dz, dz), __fmul_rn(dy, dy)), __fmul_rn(dx, dx));
-      if (d2 > g.distSqMax) continue;
-      if (slot[(int64_t)(iz >> s) * nxy + (int64_t)(iy >> s) * g.nbx + (ix >> s)] < 0) {
-        abortIdx = t;
-        break;
+  return allValue;
+}
+
+// Pass 1.  Valid particles (the marking loop's domain tests, src/msbg_demo.cpp:358-360, and
+// an owning value block: the demo walks the particle lists of value blocks only,
+// src/msbg_demo.cpp:541-566) get their abort index: the scan position (z, y, x order over
+// the box) of the first in-sphere voxel whose block is not a value block
+// (src/msbg_demo.cpp:613-618), or the box size.  Voxels from that position on are not
+// written.  Every value block the box touches counts the particle once.  abortAt = 0 marks
+// a particle that writes nothing.  A thread takes ppt particles, kListThreads apart.
+__global__ void __launch_bounds__(kListThreads) kSplatCount(const float *__restrict__ pts, int64_t n, int ppt, SplatGeom g,
+                                                            const int32_t *__restrict__ slot,
+                                                            int32_t *__restrict__ abortAt, int32_t *__restrict__ cnt,
+                                                            unsigned long long *__restrict__ nAborted) {
+  __shared__ BlockHash h;
+  hashClear(h);
+  __syncthreads();
+  const int s = g.log2bs;
+  const int64_t nxy = (int64_t)g.nbx * g.nby;
+  const int64_t first = (int64_t)blockIdx.x * ppt * kListThreads + threadIdx.x;
+  for (int q = 0; q < ppt; q++) {
+    const int64_t i = first + (int64_t)q * kListThreads;
+    if (i >= n) break;
+    const float px = pts[3 * i], py = pts[3 * i + 1], pz = pts[3 * i + 2];
+    int abortIdx = 0;
+    SplatBox b;
+    int32_t sl[8];
+    bool valid = !(px < g.domMin[0] || px > g.domMax[0] || py < g.domMin[1] || py > g.domMax[1] ||
+                   pz < g.domMin[2] || pz > g.domMax[2]);
+    if (valid) {
+      const int ix = (int)px, iy = (int)py, iz = (int)pz;
+      valid = ix >= 0 && ix < g.sx && iy >= 0 && iy < g.sy && iz >= 0 && iz < g.sz &&
+              slot[(int64_t)(iz >> s) * nxy + (int64_t)(iy >> s) * g.nbx + (ix >> s)] >= 0;
+    }
+    if (valid && splatBox(g, px, py, pz, b)) {
+      const int nx = b.ix2 - b.ix1 + 1, ny = b.iy2 - b.iy1 + 1, nz = b.iz2 - b.iz1 + 1;
+      const int total = nx * ny * nz;
+      abortIdx = total;
+      if (!boxSlots(g, b, slot, sl)) {
+        for (int t = 0; t < total; t++) {
+          const int lx = t % nx, rest = t / nx, ly = rest % ny, lz = rest / ny;
+          const int ix = b.ix1 + lx, iy = b.iy1 + ly, iz = b.iz1 + lz;
+          const float dz = __fsub_rn((float)iz, b.z0), dy = __fsub_rn((float)iy, b.y0), dx = __fsub_rn((float)ix, b.x0);
+          const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dz, dz), __fmul_rn(dy, dy)), __fmul_rn(dx, dx));
+          if (d2 > g.distSqMax) continue;
+          if (slot[(int64_t)(iz >> s) * nxy + (int64_t)(iy >> s) * g.nbx + (ix >> s)] < 0) {
+            abortIdx = t;
+            break;
+          }
+        }
+        if (abortIdx < total) atomicAdd(nAborted, 1ull);
       }
     }
-    if (abortIdx < total) atomicAdd(nAborted, 1ull);
-  }
-  abortAt[i] = abortIdx;
-  if (abortIdx == 0) return;
+    abortAt[i] = abortIdx;
+    if (abortIdx == 0) continue;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    // each distinct touched value block once
-    const bool dup = ((k & 1) && bx[1] == bx[0]) || ((k & 2) && by[1] == by[0]) || ((k & 4) && bz[1] == bz[0]);
-    if (!dup && sl[k] >= 0) atomicAdd(&cnt[sl[k]], 1);
+    for (int k = 0; k < 8; k++) {
+      if (sl[k] < 0) continue;
+      const int p = hashPlace<true>(h, sl[k]);
+      if (p >= 0) atomicAdd(&h.val[p], 1);
+      else atomicAdd(&cnt[sl[k]], 1);
+    }
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHashSize; i += kListThreads)
+    if (h.key[i] >= 0) atomicAdd(&cnt[h.key[i]], h.val[i]);
 }
 
 // Pass 2: the particle's index into the list of every value block it touches
-// (list of slot s: entries[off[s] .. off[s+1]-1], in no particular order).
-__global__ void __launch_bounds__(256) kSplatScatter(const float *__restrict__ pts, int64_t n, SplatGeom g,
-                                                     const int32_t *__restrict__ slot,
-                                                     const int32_t *__restrict__ abortAt,
-                                                     const int64_t *__restrict__ off, int32_t *__restrict__ cursor,
-                                                     int32_t *__restrict__ entries) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || abortAt[i] == 0) return;
-  const float px = pts[3 * i], py = pts[3 * i + 1], pz = pts[3 * i + 2];
-  SplatBox b;
-  splatBox(g, px, py, pz, b);
-  const int s = g.log2bs;
-  const int64_t nxy = (int64_t)g.nbx * g.nby;
-  const int bx[2] = {b.ix1 >> s, b.ix2 >> s}, by[2] = {b.iy1 >> s, b.iy2 >> s}, bz[2] = {b.iz1 >> s, b.iz2 >> s};
+// (list of slot s: entries[off[s] .. off[s+1]-1], in no particular order).  The CTA counts
+// its particles per block, reserves a run of each list, and fills it.
+__global__ void __launch_bounds__(kListThreads) kSplatScatter(const float *__restrict__ pts, int64_t n, int ppt,
+                                                              SplatGeom g, const int32_t *__restrict__ slot,
+                                                              const int32_t *__restrict__ abortAt,
+                                                              const int64_t *__restrict__ off,
+                                                              int32_t *__restrict__ cursor,
+                                                              int32_t *__restrict__ entries) {
+  __shared__ BlockHash h;
+  __shared__ int run[kHashSize];  // the CTA's first position in a block's list
+  hashClear(h);
+  __syncthreads();
+  const int64_t first = (int64_t)blockIdx.x * ppt * kListThreads + threadIdx.x;
+  auto forBlocks = [&](auto f) {
+    for (int q = 0; q < ppt; q++) {
+      const int64_t i = first + (int64_t)q * kListThreads;
+      if (i >= n) break;
+      if (abortAt[i] == 0) continue;
+      SplatBox b;
+      splatBox(g, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], b);
+      int32_t sl[8];
+      boxSlots(g, b, slot, sl);
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const bool dup = ((k & 1) && bx[1] == bx[0]) || ((k & 2) && by[1] == by[0]) || ((k & 4) && bz[1] == bz[0]);
-    if (dup) continue;
-    const int sl = slot[(int64_t)bz[k >> 2] * nxy + (int64_t)by[(k >> 1) & 1] * g.nbx + bx[k & 1]];
-    if (sl >= 0) entries[off[sl] + atomicAdd(&cursor[sl], 1)] = (int32_t)i;
-  }
+      for (int k = 0; k < 8; k++)
+        if (sl[k] >= 0) f(sl[k], (int32_t)i);
+    }
+  };
+  forBlocks([&](int sl, int32_t) {
+    const int p = hashPlace<true>(h, sl);
+    if (p >= 0) atomicAdd(&h.val[p], 1);
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHashSize; i += kListThreads)
+    if (h.key[i] >= 0) {
+      run[i] = atomicAdd(&cursor[h.key[i]], h.val[i]);
+      h.val[i] = 0;
+    }
+  __syncthreads();
+  forBlocks([&](int sl, int32_t i) {
+    const int p = hashPlace<false>(h, sl);
+    const int at = p >= 0 ? run[p] + atomicAdd(&h.val[p], 1) : atomicAdd(&cursor[sl], 1);
+    entries[off[sl] + at] = i;
+  });
 }
 
 // Pass 3, one CTA per value block (slot = blockIdx.x): the minimum of the splat
@@ -190,26 +267,18 @@ constexpr int splatThreads() { return 16 * BS; }
 template <int BS>
 constexpr int splatMinCtas() { return 1536 / splatThreads<BS>(); }
 
+// list entries a CTA takes
+template <int BS>
+constexpr int splatChunk() { return 32 * BS; }
+
+// Entries e0 .. e1-1 of a block's list into the minima of its planes Z0 .. Z0+PZ-1.
+// Bound: issue (80% of the slots).
 template <int BS, int NZ>
-__global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatBlock(const float *__restrict__ pts, SplatGeom g,
-                                                   const int32_t *__restrict__ active,
-                                                   const int32_t *__restrict__ abortAt,
-                                                   const int64_t *__restrict__ off,
-                                                   const int32_t *__restrict__ entries, const float *init,
-                                                   float *dst) {
-  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ;
-  extern __shared__ __align__(16) int smin[];
-  const int sl = blockIdx.x / NZ, zp = blockIdx.x % NZ;
-  const int bid = active[sl];
-  const int X0 = (bid % g.nbx) * BS, Y0 = ((bid / g.nbx) % g.nby) * BS,
-            Z0 = (int)(bid / ((int64_t)g.nbx * g.nby)) * BS + zp * PZ;  // this CTA's first plane
-  const int one = __float_as_int(1.0f);
-  const float *in = init ? init + (int64_t)sl * VPB + zp * VPP : nullptr;
-  for (int v = threadIdx.x; v < VPP; v += blockDim.x)
-    smin[(v / BS) * RS + v % BS] = in ? __float_as_int(in[v]) : one;
-  __syncthreads();
+__device__ __forceinline__ void splatEntries(int *smin, const float *__restrict__ pts, const SplatGeom &g, int X0, int Y0,
+                                             int Z0, const int32_t *__restrict__ abortAt,
+                                             const int32_t *__restrict__ entries, int64_t e0, int64_t e1) {
+  constexpr int RS = BS + 1, PZ = BS / NZ;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
-  const int64_t e0 = off[sl], e1 = off[sl + 1];
   for (int64_t e = e0 + warp; e < e1; e += nWarps) {
     const int i = entries[e];
     const float px = pts[3 * (int64_t)i], py = pts[3 * (int64_t)i + 1], pz = pts[3 * (int64_t)i + 2];
@@ -234,24 +303,93 @@ __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplat
       if (dzy > g.distSqMax) continue;
       const int rowScan = ((iz - b.iz1) * ny + (iy - b.iy1)) * nx - b.ix1;  // + ix: the scan index
       int *rowMin = smin + ((iz - Z0) * BS + (iy - Y0)) * RS - X0;
-      // the scan index grows with ix along the row, so the abort rule cuts the row at
-      // ab - rowScan; x runs as a float (exact for these integers)
+      // The scan index grows with ix along the row, so the abort rule cuts the row at
+      // ab - rowScan.  Two voxels a step on packed operations (splat of 768 k particles on
+      // 32^3 blocks: 960 -> 935 us), x as floats (exact for these integers); distSq exactly
+      // as the demo forms it, (dz*dz + dy*dy) + dx*dx: the square as fma(dx, dx, -0) with a
+      // run-time -0, or the compiler would fuse it into the sum.
       const int xEnd = min(cx2, ab - 1 - rowScan);
-      float fx = (float)cx1;
-      for (int ix = cx1; ix <= xEnd; ix++, fx += 1.0f) {
-        // distSq exactly as the demo forms it: (dz*dz + dy*dy) + dx*dx
-        const float dx = __fsub_rn(fx, b.x0);
-        const float d2 = __fadd_rn(dzy, __fmul_rn(dx, dx));
-        if (d2 > g.distSqMax) continue;
-        atomicMin(rowMin + ix, __float_as_int(__fmul_rn(d2, g.distSqMaxInv)));
+      float2 fx = make_float2((float)cx1, (float)(cx1 + 1));
+      const float2 nx0 = make_float2(-b.x0, -b.x0), nz = make_float2(g.negZero, g.negZero);
+      const float2 dzy2 = make_float2(dzy, dzy), inv = make_float2(g.distSqMaxInv, g.distSqMaxInv);
+#pragma unroll 1
+      for (int ix = cx1; ix <= xEnd; ix += 2) {
+        const float2 dx = __fadd2_rn(fx, nx0);
+        const float2 d2 = __fadd2_rn(dzy2, __ffma2_rn(dx, dx, nz));
+        const float2 v = __fmul2_rn(d2, inv);
+        if (d2.x <= g.distSqMax) atomicMin(rowMin + ix, __float_as_int(v.x));
+        if (d2.y <= g.distSqMax && ix < xEnd) atomicMin(rowMin + ix + 1, __float_as_int(v.y));
+        fx = __fadd2_rn(fx, make_float2(2.0f, 2.0f));
       }
     }
   }
+}
+
+// A value block's first chunk, and the write of the block.  Blocks hold very different
+// numbers of particles (a small sphere's 32,000 particles lie in a few dozen blocks), and a
+// CTA that took the longest list alone ran while the other SMs had finished: the SMs were
+// active 40% of the launch on the 512^3 workload (4.36 ms).  A longer list's other chunks
+// are queued for kSplatRest (0.34 + 1.53 ms).
+template <int BS, int NZ>
+__global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatBlock(const float *__restrict__ pts, SplatGeom g,
+                                                   const int32_t *__restrict__ active,
+                                                   const int32_t *__restrict__ abortAt,
+                                                   const int64_t *__restrict__ off,
+                                                   const int32_t *__restrict__ entries, const float *init,
+                                                   float *dst, int *__restrict__ nRest, int2 *__restrict__ rest) {
+  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ, CH = splatChunk<BS>();
+  extern __shared__ __align__(16) int smin[];
+  __shared__ int restAt;
+  const int sl = blockIdx.x / NZ, zp = blockIdx.x % NZ;
+  const int bid = active[sl];
+  const int X0 = (bid % g.nbx) * BS, Y0 = ((bid / g.nbx) % g.nby) * BS,
+            Z0 = (int)(bid / ((int64_t)g.nbx * g.nby)) * BS + zp * PZ;  // this CTA's first plane
+  const int64_t e0 = off[sl], cnt = off[sl + 1] - e0;
+  const int more = zp == 0 && cnt > CH ? (int)((cnt - 1) / CH) : 0;
+  if (more && threadIdx.x == 0) restAt = atomicAdd(nRest, more);
+  const int one = __float_as_int(1.0f);
+  const float *in = init ? init + (int64_t)sl * VPB + zp * VPP : nullptr;
+  for (int v = threadIdx.x; v < VPP; v += blockDim.x)
+    smin[(v / BS) * RS + v % BS] = in ? __float_as_int(in[v]) : one;
+  __syncthreads();
+  for (int k = threadIdx.x; k < more; k += blockDim.x) rest[restAt + k] = make_int2(sl, k + 1);
+  splatEntries<BS, NZ>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, e0 + min(cnt, (int64_t)CH));
   __syncthreads();
   float *out = dst + (int64_t)sl * VPB + zp * VPP;
   for (int v = threadIdx.x * 4; v < VPP; v += blockDim.x * 4) {
     const int *row = smin + (v / BS) * RS + v % BS;
     *reinterpret_cast<int4 *>(out + v) = make_int4(row[0], row[1], row[2], row[3]);
+  }
+}
+
+// The queued chunks: their minima are merged into the blocks that kSplatBlock has written
+// (integer minima of the bit patterns, as there).
+template <int BS, int NZ>
+__global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatRest(const float *__restrict__ pts, SplatGeom g,
+                                                   const int32_t *__restrict__ active,
+                                                   const int32_t *__restrict__ abortAt,
+                                                   const int64_t *__restrict__ off,
+                                                   const int32_t *__restrict__ entries, int *dst,
+                                                   const int *__restrict__ nRest, const int2 *__restrict__ rest) {
+  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ, CH = splatChunk<BS>();
+  extern __shared__ __align__(16) int smin[];
+  const int n = *nRest * NZ;
+  for (int w = blockIdx.x; w < n; w += gridDim.x) {
+    const int2 r = rest[w / NZ];
+    const int sl = r.x, zp = w % NZ, bid = active[sl];
+    const int X0 = (bid % g.nbx) * BS, Y0 = ((bid / g.nbx) % g.nby) * BS,
+              Z0 = (int)(bid / ((int64_t)g.nbx * g.nby)) * BS + zp * PZ;
+    for (int v = threadIdx.x; v < VPP; v += blockDim.x) smin[(v / BS) * RS + v % BS] = 0x7fffffff;
+    __syncthreads();
+    const int64_t e0 = off[sl] + (int64_t)r.y * CH;
+    splatEntries<BS, NZ>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, min(e0 + CH, off[sl + 1]));
+    __syncthreads();
+    int *out = dst + (int64_t)sl * VPB + zp * VPP;
+    for (int v = threadIdx.x; v < VPP; v += blockDim.x) {
+      const int m = smin[(v / BS) * RS + v % BS];
+      if (m != 0x7fffffff && m < __ldcg(out + v)) atomicMin(out + v, m);
+    }
+    __syncthreads();
   }
 }
 
@@ -358,44 +496,55 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
   const int64_t nn = n > 0 ? n : 1;
   const size_t bAbort = (size_t)nn * 4, bCnt = ((size_t)nAct * 4 + 15) & ~size_t(15),
                bOff = (size_t)(nAct + 1) * 8, bEnt = (size_t)nn * 8 * 4;
+  // queued chunks: fewer than the entries / the chunk length (32 bs); their count beside
+  // the list counts, which are zeroed
+  const size_t bRest = ((size_t)nn * 8 / (32 * ctx->bsx) + 1) * sizeof(int2);
   char *scratch = nullptr;
-  MSBG_CUDA(ctx, cudaMallocAsync((void **)&scratch, bAbort + 2 * bCnt + bOff + bEnt + 64, ctx->stream));
+  MSBG_CUDA(ctx, cudaMallocAsync((void **)&scratch, bAbort + 2 * bCnt + bOff + bEnt + bRest + 128, ctx->stream));
   int32_t *abortAt = (int32_t *)scratch;
   int32_t *cnt = (int32_t *)(scratch + ((bAbort + 15) & ~size_t(15)));
   int32_t *cursor = (int32_t *)((char *)cnt + bCnt);
-  int64_t *off = (int64_t *)((char *)cursor + bCnt);
-  int32_t *entries = (int32_t *)((char *)off + ((bOff + 15) & ~size_t(15)));
+  int *nRest = (int *)((char *)cursor + bCnt);
+  int64_t *off = (int64_t *)((char *)nRest + 16);
+  int2 *rest = (int2 *)((char *)off + ((bOff + 15) & ~size_t(15)));
+  int32_t *entries = (int32_t *)((char *)rest + ((bRest + 15) & ~size_t(15)));
+  // particles per thread of the list passes: more per CTA share its table, while the CTAs
+  // still fill the chip
+  const int ppt = n >= (int64_t)152 * 4 * kListThreads * 8 ? 8 : n >= (int64_t)152 * 4 * kListThreads * 2 ? 4 : 1;
+  const unsigned listGrid = gridFor(n, ppt * kListThreads);
   int rc = MSBG_GPU_OK;
   auto run = [&]() -> int {
-    MSBG_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * bCnt, ctx->stream));
+    MSBG_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * bCnt + 16, ctx->stream));
     if (n > 0) {
-      MSBG_LAUNCH(ctx, kSplatCount, gridFor(n, 256), 256, 0, dPts, n, g, ctx->dSlot, abortAt, cnt,
+      MSBG_LAUNCH(ctx, kSplatCount, listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt, cnt,
                   (unsigned long long *)(ctx->dCounters + 1));
     }
     int r = exclusiveScanCounts(ctx, cnt, nAct, off, off + nAct);
     if (r) return r;
     if (n > 0) {
-      MSBG_LAUNCH(ctx, kSplatScatter, gridFor(n, 256), 256, 0, dPts, n, g, ctx->dSlot, abortAt, off, cursor,
+      MSBG_LAUNCH(ctx, kSplatScatter, listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt, off, cursor,
                   entries);
     }
     const float *init = c.storage == MSBG_GPU_F32 ? dst : nullptr;
-    if (ctx->bsx == 32) {
-      constexpr int smem = splatSmemWords<32, 2>() * 4;
+    auto blocks = [&](auto bsC, auto nzC) -> int {
+      constexpr int BS = decltype(bsC)::value, NZ = decltype(nzC)::value, smem = splatSmemWords<BS, NZ>() * 4;
       static bool attr = false;
-      if (!attr) {
-        MSBG_CUDA(ctx, cudaFuncSetAttribute(kSplatBlock<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (smem > 48 * 1024 && !attr) {
+        MSBG_CUDA(ctx, cudaFuncSetAttribute(kSplatBlock<BS, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        MSBG_CUDA(ctx, cudaFuncSetAttribute(kSplatRest<BS, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr = true;
       }
-      MSBG_LAUNCH(ctx, (kSplatBlock<32, 2>), (unsigned)(2 * nAct), splatThreads<32>(), smem, dPts, g, ctx->dActive, abortAt, off,
-                  entries, init, dst);
-    } else if (ctx->bsx == 16) {
-      MSBG_LAUNCH(ctx, (kSplatBlock<16, 1>), (unsigned)nAct, splatThreads<16>(), (splatSmemWords<16, 1>() * 4), dPts, g, ctx->dActive,
-                  abortAt, off, entries, init, dst);
-    } else {
-      MSBG_LAUNCH(ctx, (kSplatBlock<8, 1>), (unsigned)nAct, splatThreads<8>(), (splatSmemWords<8, 1>() * 4), dPts, g, ctx->dActive,
-                  abortAt, off, entries, init, dst);
-    }
-    return MSBG_GPU_OK;
+      MSBG_LAUNCH(ctx, (kSplatBlock<BS, NZ>), (unsigned)(NZ * nAct), splatThreads<BS>(), smem, dPts, g, ctx->dActive,
+                  abortAt, off, entries, init, dst, nRest, rest);
+      if (n > splatChunk<BS>())
+        MSBG_LAUNCH(ctx, (kSplatRest<BS, NZ>), 152 * splatMinCtas<BS>(), splatThreads<BS>(), smem, dPts, g, ctx->dActive,
+                    abortAt, off, entries, (int *)dst, nRest, rest);
+      return MSBG_GPU_OK;
+    };
+    using std::integral_constant;
+    if (ctx->bsx == 32) return blocks(integral_constant<int, 32>{}, integral_constant<int, 2>{});
+    if (ctx->bsx == 16) return blocks(integral_constant<int, 16>{}, integral_constant<int, 1>{});
+    return blocks(integral_constant<int, 8>{}, integral_constant<int, 1>{});
   };
   rc = run();
   cudaFreeAsync(scratch, ctx->stream);
