@@ -338,21 +338,41 @@ __global__ void kBlockFlags(const int32_t *__restrict__ levels, uint16_t *__rest
   if (level >= 0 && level < 8) atomicAdd(&perLevel[level], 1ull);
 }
 
-__global__ void kValueFlags(const int32_t *__restrict__ levels, int64_t n, int32_t *__restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = levels[i] == 0;
+// Slots of the value blocks (level 0): the exclusive scan's three kernels over (level == 0),
+// the last of which writes slot[bid] (-1 for other blocks) and the active list itself.
+__global__ void __launch_bounds__(kScanThreads) kSlotReduce(const int32_t *__restrict__ levels, int64_t n,
+                                                            int64_t *__restrict__ part) {
+  const int64_t base = (int64_t)blockIdx.x * kScanTile;
+  int64_t s = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    const int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
+    if (i < n) s += levels[i] == 0;
+  }
+  int64_t tot;
+  blockExclusive(s, &tot);
+  if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-// slot[bid] = exclusive-scan offset for value blocks, -1 otherwise; active list.
-__global__ void kAssignSlots(const int32_t *__restrict__ levels, const int64_t *__restrict__ off,
-                             int64_t n, int32_t *__restrict__ slot, int32_t *__restrict__ active) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (levels[i] == 0) {
-    slot[i] = (int32_t)off[i];
-    active[off[i]] = (int32_t)i;
-  } else {
-    slot[i] = -1;
+// part: the tiles' first slots
+__global__ void __launch_bounds__(kScanThreads) kSlotApply(const int32_t *__restrict__ levels, int64_t n,
+                                                           const int64_t *__restrict__ part, int32_t *__restrict__ slot,
+                                                           int32_t *__restrict__ active) {
+  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  bool v[kScanItems];
+  int64_t s = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    v[k] = base + k < n && levels[base + k] == 0;
+    s += v[k];
+  }
+  int64_t tot;
+  int64_t at = blockExclusive(s, &tot) + part[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    if (base + k >= n) break;
+    slot[base + k] = v[k] ? (int32_t)at : -1;
+    if (v[k]) active[at++] = (int32_t)(base + k);
   }
 }
 
@@ -360,25 +380,86 @@ __device__ __forceinline__ int blockColor8(int bx, int by, int bz) {
   return (bx & 1) + ((by & 1) << 1) + ((bz & 1) << 2);  // src/msbg.h:642-646
 }
 
-__global__ void kColorFlags(const int32_t *__restrict__ active, int64_t nAct, int nbx, int nby, int color,
-                            int32_t *__restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nAct) return;
-  const int bid = active[i];
-  const int bx = bid % nbx, by = (bid / nbx) % nby, bz = bid / (nbx * nby);
-  out[i] = blockColor8(bx, by, bz) == color;
+// The 8-colour lists: the active list's blocks by colour, each colour in ascending order, as
+// one stable partition.  Eight counts of at most 4,096 (a tile's blocks) fit two int64s in
+// 16-bit fields, so the scan of an int64 serves four colours.  The kernels read the active
+// count from the device, so that the host reads the layout's counts once, at the end.
+// (One compaction per colour took 40 launches and a second read-back: about 100 us of a
+// 64^3 frame.)
+struct ColorCounts {
+  int64_t lo, hi;  // colours 0..3 and 4..7
+};
+__device__ __forceinline__ void colorAdd(ColorCounts &c, int color) {
+  const int64_t one = 1ll << (16 * (color & 3));
+  if (color < 4) c.lo += one; else c.hi += one;
+}
+__device__ __forceinline__ int colorGet(const ColorCounts &c, int color) {
+  return (int)(((color < 4 ? c.lo : c.hi) >> (16 * (color & 3))) & 0xffff);
+}
+__device__ __forceinline__ int colorOf(int bid, int nbx, int nby) {
+  return blockColor8(bid % nbx, (bid / nbx) % nby, bid / (nbx * nby));
 }
 
-// The colour's list starts after the lists of the lower colours, whose lengths the
-// earlier scans left in colTot[0..color-1] on the device.
-__global__ void kColorScatter(const int32_t *__restrict__ active, const int32_t *__restrict__ flag,
-                              const int64_t *__restrict__ off, int64_t nAct, const int64_t *__restrict__ colTot,
-                              int color, int32_t *__restrict__ colorBids) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nAct || !flag[i]) return;
-  int64_t base = 0;
-  for (int c = 0; c < color; c++) base += colTot[c];
-  colorBids[base + off[i]] = active[i];
+// part[tile][8]: blocks of each colour in the tile
+__global__ void __launch_bounds__(kScanThreads) kColorReduce(const int32_t *__restrict__ active,
+                                                             const int64_t *__restrict__ nActPtr, int nbx, int nby,
+                                                             int32_t *__restrict__ part) {
+  const int64_t nAct = *nActPtr, base = (int64_t)blockIdx.x * kScanTile;
+  ColorCounts c{0, 0}, tot;
+  for (int k = 0; k < kScanItems; k++) {
+    const int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
+    if (i < nAct) colorAdd(c, colorOf(active[i], nbx, nby));
+  }
+  blockExclusive(c.lo, &tot.lo);
+  blockExclusive(c.hi, &tot.hi);
+  if (threadIdx.x < 8) part[(int64_t)blockIdx.x * 8 + threadIdx.x] = colorGet(tot, threadIdx.x);
+}
+
+// part <- first position of the tile's blocks of each colour in colorBids; colTot: the colours' sizes
+__global__ void __launch_bounds__(kScanThreads) kColorPartials(int32_t *__restrict__ part, int64_t nTiles,
+                                                               int64_t *__restrict__ colTot) {
+  int64_t start = 0;
+  for (int color = 0; color < 8; color++) {
+    int64_t carry = 0;
+    for (int64_t t0 = 0; t0 < nTiles; t0 += kScanThreads) {
+      const int64_t t = t0 + threadIdx.x;
+      const int64_t v = t < nTiles ? part[t * 8 + color] : 0;
+      int64_t tot;
+      const int64_t ex = blockExclusive(v, &tot);
+      if (t < nTiles) part[t * 8 + color] = (int32_t)(start + carry + ex);
+      carry += tot;
+    }
+    if (threadIdx.x == 0) colTot[color] = carry;
+    start += carry;
+  }
+}
+
+__global__ void __launch_bounds__(kScanThreads) kColorApply(const int32_t *__restrict__ active,
+                                                            const int64_t *__restrict__ nActPtr, int nbx, int nby,
+                                                            const int32_t *__restrict__ part,
+                                                            int32_t *__restrict__ colorBids) {
+  const int64_t nAct = *nActPtr, base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  if ((int64_t)blockIdx.x * kScanTile >= nAct) return;
+  int bid[kScanItems], color[kScanItems];
+  ColorCounts c{0, 0}, tot;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    color[k] = -1;
+    if (base + k < nAct) {
+      bid[k] = active[base + k];
+      color[k] = colorOf(bid[k], nbx, nby);
+      colorAdd(c, color[k]);
+    }
+  }
+  ColorCounts ex;
+  ex.lo = blockExclusive(c.lo, &tot.lo);
+  ex.hi = blockExclusive(c.hi, &tot.hi);
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    if (color[k] < 0) continue;
+    colorBids[part[(int64_t)blockIdx.x * 8 + color[k]] + colorGet(ex, color[k])] = bid[k];
+    colorAdd(ex, color[k]);
+  }
 }
 
 }  // namespace msbg
@@ -635,43 +716,36 @@ extern "C" int msbg_gpu_set_refinement_map(msbg_gpu_ctx *ctx, double fillValue) 
   MSBG_CUDA(ctx, cudaMemsetAsync(dCnt + 4, 0, 8 * 8, ctx->stream));
   MSBG_LAUNCH(ctx, kBlockFlags, gridFor(nB, 256), 256, 0, ctx->dLevels, ctx->dFlags, ctx->nbx,
               ctx->nby, ctx->nbz, (unsigned long long *)(dCnt + 4));
-  // slot assignment: scan of (level == 0) over all blocks; dLevelsTmp holds the flags,
-  // the int64 offsets go to the tmp slab.
-  int rc = ensureTmpSlab(ctx, (size_t)nB * 8);
-  if (rc) return rc;
-  int64_t *dOff = (int64_t *)ctx->dTmpSlab;
-  MSBG_LAUNCH(ctx, kValueFlags, gridFor(nB, 256), 256, 0, ctx->dLevels, nB, ctx->dLevelsTmp);
-  rc = exclusiveScanFlags(ctx, ctx->dLevelsTmp, nB, dOff, dCnt + 2);
-  if (rc) return rc;
-  MSBG_LAUNCH(ctx, kAssignSlots, gridFor(nB, 256), 256, 0, ctx->dLevels, dOff, nB, ctx->dSlot,
+  // slots and the active list, then the 8-colour lists (their partial counts in
+  // dLevelsTmp: 8 per tile of 4,096 blocks); one read-back of all counts
+  const int64_t nTiles = (nB + kScanTile - 1) / kScanTile;
+  int64_t *dColTot = dCnt + kColorTot;
+  int rc;
+  int32_t *colorPart = nB >= 8 * nTiles ? ctx->dLevelsTmp : nullptr;
+  if (!colorPart) {  // fewer than 8 blocks
+    if ((rc = ensureTmpSlab(ctx, (size_t)nTiles * 8 * 4))) return rc;
+    colorPart = (int32_t *)ctx->dTmpSlab;
+  }
+  MSBG_LAUNCH(ctx, kSlotReduce, (unsigned)nTiles, kScanThreads, 0, ctx->dLevels, nB, ctx->dScanPartial);
+  MSBG_LAUNCH(ctx, kScanPartials, 1, kScanThreads, 0, ctx->dScanPartial, nTiles, dCnt + 2);
+  MSBG_LAUNCH(ctx, kSlotApply, (unsigned)nTiles, kScanThreads, 0, ctx->dLevels, nB, ctx->dScanPartial, ctx->dSlot,
               ctx->dActive);
-  if ((rc = readSmall(ctx, ctx->hCounters, dCnt, 16 * 8))) return rc;  // 0..15
+  MSBG_LAUNCH(ctx, kColorReduce, (unsigned)nTiles, kScanThreads, 0, ctx->dActive, dCnt + 2, ctx->nbx, ctx->nby,
+              colorPart);
+  MSBG_LAUNCH(ctx, kColorPartials, 1, kScanThreads, 0, colorPart, nTiles, dColTot);
+  MSBG_LAUNCH(ctx, kColorApply, (unsigned)nTiles, kScanThreads, 0, ctx->dActive, dCnt + 2, ctx->nbx, ctx->nby, colorPart,
+              ctx->dColorBids);
+  if ((rc = readSmall(ctx, ctx->hCounters, dCnt, (kColorTot + 8) * 8))) return rc;
   const int64_t nAct = ctx->hCounters[2];
   for (int l = 0; l < 8; l++) ctx->blocksPerLevel[l] = ctx->hCounters[4 + l];
   ctx->nActParticles = ctx->hCounters[0];
   if (nAct > ctx->capacityLimit)
     return fail(ctx, MSBG_GPU_ERR_CAPACITY, "%lld value blocks exceed the pool capacity %lld",
                 (long long)nAct, (long long)ctx->capacityLimit);
-  // 8-color lists: stable compaction of the active list per color; each colour's
-  // length stays on the device (counters kColorTot..+7), where the next colours'
-  // scatters read their start, and all eight are read back once.
-  int32_t *dFlag = ctx->dLevelsTmp;
-  int64_t *dColTot = dCnt + kColorTot;
-  if (nAct > 0) {
-    for (int c = 0; c < 8; c++) {
-      MSBG_LAUNCH(ctx, kColorFlags, gridFor(nAct, 256), 256, 0, ctx->dActive, nAct, ctx->nbx, ctx->nby,
-                  c, dFlag);
-      rc = exclusiveScanFlags(ctx, dFlag, nAct, dOff, dColTot + c);
-      if (rc) return rc;
-      MSBG_LAUNCH(ctx, kColorScatter, gridFor(nAct, 256), 256, 0, ctx->dActive, dFlag, dOff, nAct, dColTot,
-                  c, ctx->dColorBids);
-    }
-    if ((rc = readSmall(ctx, ctx->hCounters + kColorTot, dColTot, 8 * 8))) return rc;
-  }
   int32_t base = 0;
   for (int c = 0; c < 8; c++) {
     ctx->colorStart[c] = base;
-    if (nAct > 0) base += (int32_t)ctx->hCounters[kColorTot + c];
+    base += (int32_t)ctx->hCounters[kColorTot + c];
   }
   ctx->colorStart[8] = base;
   ctx->nActive = nAct;
