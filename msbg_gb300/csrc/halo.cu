@@ -23,6 +23,7 @@
 //
 // Bytes per block: bs^3 S own reads + the halo's neighbour reads, (bs+2h)^3 * 4 written.
 #include <math.h>
+#include <string.h>
 
 #include "internal.cuh"
 
@@ -81,6 +82,7 @@ struct HaloArgs {
   int sx, sy, sz;         // level-l domain
   int nbx, nby, nbz;
   int opt;
+  int quadOk, pairOk;     // kFillHaloRows: level l (l+1) payload aligned to 4 (2) elements
   float *out;
   unsigned long long *skipped;
 };
@@ -247,6 +249,229 @@ __global__ void __launch_bounds__(kHaloThreads, 8) kFillHalo(HaloArgs a) {
   }
 }
 
+// The same boxes by rows, for block edges of 8 and more: one CTA per block, and each of its
+// warps on its own.  Two box planes are hs / 2 groups of four rows; a warp keeps one group
+// and goes through the plane pairs, so what a lane reads, one quad of four voxels above the
+// block and one voxel of the halo columns, moves by a constant from pair to pair while the
+// plane lies in the block.  Only in the planes below and above, and in the first two planes
+// of the block, a lane looks its source up: in a table of the 27 blocks around, which holds
+// payload, mask and replacement of the local coordinates (a clamp to the block's face) and
+// the level.  Edges 16 and 8 put two and four plane pairs side by side in a warp.  The four
+// rows leave together: whole 16-byte stores, whole sectors.  The next pair's loads fly
+// meanwhile, and nothing in the CTA waits for another warp.
+// The plane-wise form above resolves every shell position of every plane and has a barrier
+// per plane; looking every row up (the table, but no constant step) was bound by issue as
+// well, 87 k warp instructions a block against 37 k.  Measured (FP16, bs 32, halo 1, a
+// coarser level beside, 2,565 blocks, 540 MB): 233 us plane-wise, 236 with every row looked
+// up, 190 so; bound now by the loads' latency (45% of issue slots, 30 warps per SM).
+template <typename T>
+struct HaloEntry {
+  const T *p;           // null: the constant c
+  uint32_t mask, repl;  // of the packed local coordinates x | y << 10 | z << 20
+  float c;
+  int sh;               // 1: p is at level l+1
+};
+
+template <typename T>
+__device__ __forceinline__ HaloEntry<T> haloEntry(const HaloArgs &a, const int32_t *stL, const int32_t *stC, int bx,
+                                                  int by, int bz, int n) {
+  const int bs = a.bs;
+  const int d[3] = {n % 3 - 1, (n / 3) % 3 - 1, n / 9 - 1}, b[3] = {bx + d[0], by + d[1], bz + d[2]};
+  const int nb[3] = {a.nbx, a.nby, a.nbz};
+  HaloEntry<T> e{nullptr, 0x3fffffffu, 0u, a.lv.emptyF, 0};
+  auto clamp = [&](int k) {  // axis k to the face of the block through which it leaves
+    e.mask &= ~(1023u << (10 * k));
+    if (d[k] > 0) e.repl |= (uint32_t)(bs - 1) << (10 * k);
+  };
+  auto take = [&](const HaloLevel &L, int32_t st, int edge, int sh) {
+    if (st >= 0) e.p = (const T *)L.pay + (int64_t)st * edge * edge * edge;
+    else e.c = st == MSBG_GPU_LBLK_EMPTY ? L.emptyF : L.fullF;
+    e.sh = sh;
+  };
+  if (stL[n] != MSBG_GPU_LBLK_NONE) {  // in the domain, and the block exists
+    take(a.lv, stL[n], bs, 0);
+  } else if (a.opt & MSBG_GPU_BC_NEUMANN) {
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      if (d[k]) clamp(k);
+    take(a.lv, stL[13], bs, 0);
+  } else if (a.opt & MSBG_GPU_BC_COARSE_LEVEL) {
+    int nc = 0, pw = 1;
+    bool inRange = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++, pw *= 3) {  // axes outside the domain go back to it
+      const bool in = b[k] >= 0 && b[k] < nb[k];
+      if (!in) clamp(k);
+      inRange = inRange && in;
+      nc += pw * (in ? d[k] + 1 : 1);
+    }
+    if (!inRange && stL[nc] != MSBG_GPU_LBLK_NONE) take(a.lv, stL[nc], bs, 0);
+    else if (stC[nc] != MSBG_GPU_LBLK_NONE) take(a.lo, stC[nc], bs >> 1, 1);
+  }
+  return e;
+}
+
+template <typename T> struct HaloRaw { uint2 q; };
+template <> struct HaloRaw<float> { float4 q; };
+
+constexpr int kHaloRowThreads = 288;  // 17 groups (bs 32, halo 1) in two rounds
+template <typename T, int L>
+__global__ void __launch_bounds__(kHaloRowThreads, 4) kFillHaloRows(HaloArgs a) {
+  constexpr int BS = 1 << L, PR = BS / 4, M = BS - 1;  // quads per row
+  constexpr int NP = 32 / (4 * PR), LP = 32 / NP;      // plane pairs side by side, lanes of each
+  __shared__ int32_t stL[27], stC[27];
+  __shared__ HaloEntry<T> tab[27];
+  extern __shared__ __align__(16) float staging[];
+  const int bid = a.bids[blockIdx.x];
+  const int64_t nxy = (int64_t)a.nbx * a.nby;
+  const int64_t nBlocks = nxy * a.nbz;
+  if (bid < 0 || bid >= nBlocks || a.levels[bid] != a.level || !a.lv.state ||
+      a.lv.state[bid] == MSBG_GPU_LBLK_NONE) {
+    if (threadIdx.x == 0) atomicAdd(a.skipped, 1ull);
+    return;
+  }
+  const int bx = (int)(bid % a.nbx), by = (int)((bid / a.nbx) % a.nby), bz = (int)(bid / nxy);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid < 27) {
+    const int x = bx + tid % 3 - 1, y = by + (tid / 3) % 3 - 1, z = bz + tid / 9 - 1;
+    int32_t l = MSBG_GPU_LBLK_NONE, c = MSBG_GPU_LBLK_NONE;
+    if (x >= 0 && y >= 0 && z >= 0 && x < a.nbx && y < a.nby && z < a.nbz) {
+      const int64_t b = (int64_t)z * nxy + (int64_t)y * a.nbx + x;
+      l = a.lv.state[b];
+      if (a.lo.state) c = a.lo.state[b];
+    }
+    stL[tid] = l;
+    stC[tid] = c;
+  }
+  __syncthreads();
+  if (tid < 27) tab[tid] = haloEntry<T>(a, stL, stC, bx, by, bz, tid);
+  __syncthreads();
+  const int h = a.h, hs = a.hs, side = 2 * h, nPair = hs / 2;
+  const int part = lane / LP, sub = lane % LP;  // plane pair of the warp's NP, lane within it
+  float *const staged = staging + wid * NP * 4 * hs, *const st = staged + part * 4 * hs;
+  for (int group = wid; group < nPair; group += kHaloRowThreads / 32) {
+    float *dst = a.out + (int64_t)blockIdx.x * hs * hs * hs + 4 * group * hs;  // + 2 hs^2 per plane pair
+    // what a lane reads now: kind 0 the constant c, 1 p, 2 p at the coarser level
+    struct Stream {
+      const T *p;
+      float c;
+      int kind;
+    };
+    auto seek = [&](Stream &s, int hx, int hy, int z) {
+      const int x = hx - h, y = hy - h;
+      const HaloEntry<T> &e = tab[((x >> L) + 1) + 3 * ((y >> L) + 1) + 9 * ((z >> L) + 1)];
+      const uint32_t loc = (((uint32_t)(x & M) | (uint32_t)(y & M) << 10 | (uint32_t)(z & M) << 20) & e.mask) | e.repl;
+      const int sh = e.sh, l2 = L - sh;
+      s.p = e.p + (((((int)(loc >> 20) >> sh) << l2) + ((int)(loc >> 10 & 1023) >> sh)) << l2) + ((int)(loc & 1023) >> sh);
+      s.c = e.c;
+      s.kind = e.p ? 1 + sh : 0;
+    };
+    // this lane's quad and halo column: row of the two planes' 2 hs, plane of the two, column
+    const int rq = 4 * group + sub / PR, zq = rq >= hs, yq = rq - zq * hs, xq = h + 4 * (sub % PR);
+    const bool hasS = sub < 4 * side;
+    const int rs = 4 * group + (hasS ? sub / side : 0), zs = rs >= hs, ys = rs - zs * hs;
+    const int xs = (sub % side) < h ? sub % side : sub % side + BS;
+    Stream sq{nullptr, 0.0f, 0}, ss{nullptr, 0.0f, 0};
+    // two plane pairs in flight
+    struct Slot {
+      HaloRaw<T> q;  // a quad's voxels, two coarse voxels, or the constant's bits
+      uint32_t s;    // the halo column's voxel or constant
+      int kinds;     // of the quad | of the column << 2
+    };
+    auto issue = [&](int k, Slot &t) {  // plane pair k of this lane; called for k, k + NP, ...
+      if (k >= nPair) return;
+      auto at = [&](Stream &s, int hx, int hy, int hz) {
+        const int z = hz - h;
+        if (z < 2 * NP || z >= BS) seek(s, hx, hy, z);  // the block's first pair may be any of NP
+        else s.p += s.kind == 2 ? NP * BS * BS / 4 : NP * 2 * BS * BS;  // 2 NP planes, half as many coarse ones
+      };
+      at(sq, xq, yq, 2 * k + zq);
+      if (sq.kind == 1) {
+        if (a.quadOk) {
+          if constexpr (sizeof(T) == 4) t.q.q = __ldg(reinterpret_cast<const float4 *>(sq.p));
+          else t.q.q = __ldg(reinterpret_cast<const uint2 *>(sq.p));
+        } else {
+          T v[4] = {sq.p[0], sq.p[1], sq.p[2], sq.p[3]};
+          memcpy(&t.q, v, sizeof(v));
+        }
+      } else if (sq.kind == 2) {
+        T v[2];
+        if (a.pairOk) {
+          if constexpr (sizeof(T) == 4) { const float2 w = __ldg(reinterpret_cast<const float2 *>(sq.p)); memcpy(v, &w, 8); }
+          else { const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(sq.p)); memcpy(v, &w, 4); }
+        } else {
+          v[0] = sq.p[0];
+          v[1] = sq.p[1];
+        }
+        memcpy(&t.q, v, sizeof(v));
+      } else {
+        memcpy(&t.q, &sq.c, 4);
+      }
+      if (hasS) {
+        at(ss, xs, ys, 2 * k + zs);
+        if (ss.kind) {
+          const T v = *ss.p;
+          t.s = 0;
+          memcpy(&t.s, &v, sizeof(T));
+        } else {
+          memcpy(&t.s, &ss.c, 4);
+        }
+      }
+      t.kinds = sq.kind | ss.kind << 2;
+    };
+    auto write = [&](int k0, const Slot &t) {
+      if (k0 + part < nPair) {
+        float f[4];
+        T v[4];
+        memcpy(v, &t.q, sizeof(v));
+        if ((t.kinds & 3) == 1) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) f[i] = Store<T>::load(v + i);
+        } else if ((t.kinds & 3) == 2) {
+          f[0] = f[1] = Store<T>::load(v);
+          f[2] = f[3] = Store<T>::load(v + 1);
+        } else {
+          memcpy(f, &t.q, 4);
+          f[1] = f[2] = f[3] = f[0];
+        }
+        float *o = st + (sub / PR) * hs + xq;
+        o[0] = f[0]; o[1] = f[1]; o[2] = f[2]; o[3] = f[3];
+        if (hasS) {
+          T w;
+          memcpy(&w, &t.s, sizeof(T));
+          st[(rs - 4 * group) * hs + xs] = t.kinds >> 2 ? Store<T>::load(&w) : __uint_as_float(t.s);
+        }
+      }
+    };
+    const int pairF4 = hs * hs / 2;  // 16-byte stores per plane pair
+    auto out = [&](int k0) {
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < NP; q++) {
+        if (k0 + q >= nPair) break;
+        float4 *o4 = reinterpret_cast<float4 *>(dst) + (k0 + q) * pairF4;
+        const float4 *b4 = reinterpret_cast<const float4 *>(staged + q * 4 * hs);
+        if (lane < hs) o4[lane] = b4[lane];
+        if (lane + 32 < hs) o4[lane + 32] = b4[lane + 32];  // hs <= 40
+      }
+      __syncwarp();
+    };
+    Slot ta, tb;
+    issue(part, ta);
+    issue(part + NP, tb);
+#pragma unroll 1
+    for (int k0 = 0; k0 < nPair; k0 += 2 * NP) {
+      write(k0, ta);
+      issue(k0 + part + 2 * NP, ta);
+      out(k0);
+      if (k0 + NP >= nPair) break;
+      write(k0 + NP, tb);
+      issue(k0 + part + 3 * NP, tb);
+      out(k0 + NP);
+    }
+  }
+}
+
 // Restriction of halo boxes ((bs+2)^3, halo 1) to (bs/2)^3 coarse values: the 4^3
 // Gauss-like weights (1,3,3,1)^3/512 (src/grid.c:30-70) in the reference's summation
 // order (per x offset i and row j, S[j][i] = fma(w, f, S[j][i]) over the 4 planes; then
@@ -304,6 +529,22 @@ float quantConst(int storage, float v) {
     case MSBG_GPU_F16: return __half2float(__float2half_rn(v));
     default: return v;
   }
+}
+
+// Rows of quads need block edges of 8, and lanes for the four rows' halo columns (8 h of
+// them, beside bs quads); other boxes go plane by plane.
+template <typename T>
+int fillHaloLaunch(msbg_gpu_ctx *ctx, HaloArgs a, int64_t n, size_t smem) {
+  // caller arrays may be aligned to their elements only
+  a.quadOk = ((uintptr_t)a.lv.pay & (4 * sizeof(T) - 1)) == 0;
+  a.pairOk = ((uintptr_t)a.lo.pay & (2 * sizeof(T) - 1)) == 0;
+  const size_t rows = (size_t)(kHaloRowThreads / 32) * (a.bs >= 8 ? 32 / a.bs : 0) * 4 * a.hs * sizeof(float);
+  const unsigned nt = kHaloRowThreads;
+  if (a.bs < 8 || 8 * a.h > a.bs) MSBG_LAUNCH(ctx, kFillHalo<T>, (unsigned)n, kHaloThreads, smem, a);
+  else if (a.bs == 32) MSBG_LAUNCH(ctx, (kFillHaloRows<T, 5>), (unsigned)n, nt, rows, a);
+  else if (a.bs == 16) MSBG_LAUNCH(ctx, (kFillHaloRows<T, 4>), (unsigned)n, nt, rows, a);
+  else MSBG_LAUNCH(ctx, (kFillHaloRows<T, 3>), (unsigned)n, nt, rows, a);
+  return MSBG_GPU_OK;
 }
 
 LevelChannels *levelChannels(msbg_gpu_ctx *ctx) {
@@ -436,11 +677,13 @@ extern "C" int msbg_gpu_fill_halo_blocks(msbg_gpu_ctx *ctx, int lchan, int level
   a.skipped = lc->dSkip;
   const size_t smem = 2 * sizeof(float) * (size_t)a.hs * a.hs;  // the plane double buffer (<= 12.8 KB)
   if (n > 0) {
+    int rc;
     switch (c.storage) {
-      case MSBG_GPU_F32: MSBG_LAUNCH(ctx, kFillHalo<float>, (unsigned)n, kHaloThreads, smem, a); break;
-      case MSBG_GPU_F16: MSBG_LAUNCH(ctx, kFillHalo<__half>, (unsigned)n, kHaloThreads, smem, a); break;
-      default: MSBG_LAUNCH(ctx, kFillHalo<uint16_t>, (unsigned)n, kHaloThreads, smem, a); break;
+      case MSBG_GPU_F32: rc = fillHaloLaunch<float>(ctx, a, n, smem); break;
+      case MSBG_GPU_F16: rc = fillHaloLaunch<__half>(ctx, a, n, smem); break;
+      default: rc = fillHaloLaunch<uint16_t>(ctx, a, n, smem); break;
     }
+    if (rc) return rc;
   }
   if (hSkipped) {
     unsigned long long s = 0;
