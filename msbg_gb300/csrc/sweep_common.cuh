@@ -201,6 +201,43 @@ __device__ __forceinline__ void loadPlane(const float *row0, PlaneMcfX &P) {
   P.h5 = __fmul_rn(0.5f, __fsub_rn(row0[2 * RS + 5], row0[5]));
 }
 
+// The same planes from a thread's own three rows (four values each: y-1, y, y+1) and, in the
+// lanes that hold a block row's first and last strip (edge), one value beyond it per row;
+// the other lanes' values beyond the strip are their neighbours' (a row's strips lie in
+// consecutive lanes).
+struct StripRows {
+  float m[4], c[4], p[4], em, ec, ep;
+};
+__device__ __forceinline__ void sides(float first, float last, float beyond, bool atFirst, bool atLast, float &left,
+                                      float &right) {
+  const float l = __shfl_up_sync(0xffffffffu, last, 1), r = __shfl_down_sync(0xffffffffu, first, 1);
+  left = atFirst ? beyond : l;
+  right = atLast ? beyond : r;
+}
+__device__ __forceinline__ void planeOf(const StripRows &s, bool atFirst, bool atLast, PlaneJac &P) {
+  P.r1[1] = s.c[0]; P.r1[2] = s.c[1]; P.r1[3] = s.c[2]; P.r1[4] = s.c[3];
+  sides(s.c[0], s.c[3], s.ec, atFirst, atLast, P.r1[0], P.r1[5]);
+  const float2 s01 = add2(pr(s.m[0], s.m[1]), pr(s.p[0], s.p[1])), s23 = add2(pr(s.m[2], s.m[3]), pr(s.p[2], s.p[3]));
+  P.sy[0] = s01.x; P.sy[1] = s01.y; P.sy[2] = s23.x; P.sy[3] = s23.y;
+}
+__device__ __forceinline__ void planeOf(const StripRows &s, bool atFirst, bool atLast, PlaneMcf &P) {
+  P.r1[1] = s.c[0]; P.r1[2] = s.c[1]; P.r1[3] = s.c[2]; P.r1[4] = s.c[3];
+  sides(s.c[0], s.c[3], s.ec, atFirst, atLast, P.r1[0], P.r1[5]);
+  const float2 d01 = sub2(pr(s.p[0], s.p[1]), pr(s.m[0], s.m[1])), d23 = sub2(pr(s.p[2], s.p[3]), pr(s.m[2], s.m[3]));
+  const float2 s01 = add2(pr(s.m[0], s.m[1]), pr(s.p[0], s.p[1])), s23 = add2(pr(s.m[2], s.m[3]), pr(s.p[2], s.p[3]));
+  P.dy[1] = d01.x; P.dy[2] = d01.y; P.dy[3] = d23.x; P.dy[4] = d23.y;
+  sides(d01.x, d23.y, s.ep - s.em, atFirst, atLast, P.dy[0], P.dy[5]);
+  P.sy[0] = s01.x; P.sy[1] = s01.y; P.sy[2] = s23.x; P.sy[3] = s23.y;
+}
+__device__ __forceinline__ void planeOf(const StripRows &s, bool atFirst, bool atLast, PlaneMcfX &P) {
+  P.r1[1] = s.c[0]; P.r1[2] = s.c[1]; P.r1[3] = s.c[2]; P.r1[4] = s.c[3];
+  sides(s.c[0], s.c[3], s.ec, atFirst, atLast, P.r1[0], P.r1[5]);
+#pragma unroll
+  for (int i = 0; i < 4; i++) { P.r0[i] = s.m[i]; P.r2[i] = s.p[i]; }
+  sides(__fmul_rn(0.5f, __fsub_rn(s.p[0], s.m[0])), __fmul_rn(0.5f, __fsub_rn(s.p[3], s.m[3])),
+        __fmul_rn(0.5f, __fsub_rn(s.ep, s.em)), atFirst, atLast, P.h0, P.h5);
+}
+
 // 1/x from the hardware's approximate reciprocal (PTX rcp.approx.ftz.f32).
 __device__ __forceinline__ float rcpApprox(float x) {
   float r;
