@@ -26,6 +26,7 @@
 // call.  Same-color blocks are never 26-neighbours, so in a pass no block reads
 // a cache entry that the pass writes.  Every piece is a multiple of 16 bytes at
 // a 16-byte aligned address, as cp.async.bulk requires.
+#include <stddef.h>
 #include <string.h>
 
 #include <type_traits>
@@ -97,12 +98,13 @@ struct ColorSweep {
 template <typename T, int BS>
 struct RawTile {
   T blk[BS * BS * BS];   // own block [z][y][x]
-  T zpl[2][BS * BS];     // plane z=-1 (0) and z=BS (1), [y][x]
   T xf[2][BS * BS];      // column x=-1 (0) and x=BS (1), [z][y]
   T yr[2][BS * BS];      // row y=-1 (0) and y=BS (1), [z][x]
+  alignas(16) T er[16];  // the empty value (source of every fill from an empty block)
+  // from here on not staged by the direct 7-point form (facesOnly)
+  T zpl[2][BS * BS];     // plane z=-1 (0) and z=BS (1), [y][x]
   T cn[4][BS];           // corner columns (x=-1|BS, y=-1|BS), k = (dx>0) + 2*(dy>0), [z]
   T zh[2][4][BS];        // planes -1 / BS: x=-1 row, x=BS row (over y), y=-1 row, y=BS row (over x)
-  alignas(16) T er[16];  // the empty value (source of every fill from an empty block)
 };
 
 __device__ __forceinline__ uint32_t smemAddr(const void *p) {
@@ -153,10 +155,22 @@ struct ColorArgs {
   SweepParams p;
 };
 
+// Stencil forms that read FP16 rows straight from the staged tile (see kSweepColor).
+template <typename T, int FK>
+constexpr bool directRows() { return std::is_same<T, __half>::value && FK != 0; }
+
+// The direct 7-point form: a thread needs its own four voxels of the planes z=-1 and z=BS, which
+// it reads from global memory, and no corner.  Without those pieces (4.9 KB) three CTAs of a
+// 32^3 block share an SM (72 registers): 514 M voxels, 10 iterations, 6.12 -> 4.92 ms.  The same
+// for the direct MCF form (80 registers, planes from global memory) was slower on 102 M voxels,
+// 2.51 -> 2.66 ms.
+template <typename T, int FK>
+constexpr bool facesOnly() { return directRows<T, FK>() && (FK & ~FK_CLAMP) == K_JACOBI; }
+
 // Copy slot c of chunk k (planes k*CZ .. k*CZ+CZ-1) of a block's tile: fills
 // (dst, src, bytes) and returns true when the piece exists (its source block is a
 // value block).  Chunk 0 also carries plane z=-1, the last chunk plane z=BS.
-template <typename T, int BS>
+template <typename T, int BS, int FK>
 __device__ __forceinline__ bool tileCopy(int k, int c, const int *nbs, const ColorArgs &a,
                                          RawTile<T, BS> &t, void *&dst, const void *&src,
                                          uint32_t &bytes) {
@@ -194,6 +208,7 @@ __device__ __forceinline__ bool tileCopy(int k, int c, const int *nbs, const Col
     return true;
   }
   c -= 2 * CZ;
+  if constexpr (facesOnly<T, FK>()) return false;
   if (c < 4) {  // corner-column segments of the 4 diagonal neighbours in the block's z-layer
     const int dx = (c & 1) ? 1 : -1, dy = (c & 2) ? 1 : -1;
     const int s = NB(dx, dy, 0);
@@ -242,12 +257,10 @@ constexpr size_t rawTileBytes() {
   return (sizeof(RawTile<T, BS>) + 15) & ~size_t(15);
 }
 
-// Stencil forms that read FP16 rows straight from the staged tile (see kSweepColor).
-template <typename T, int FK>
-constexpr bool directRows() { return std::is_same<T, __half>::value && FK != 0; }
-
 template <typename T, int BS, int FK, int ZG>
 constexpr size_t colorSmemBytes() {
+  using Tile = RawTile<T, BS>;
+  if (facesOnly<T, FK>()) return offsetof(Tile, zpl);
   if (directRows<T, FK>()) return rawTileBytes<T, BS>();
   return rawTileBytes<T, BS>() + 2 * sizeof(float) * ColorSweep<T, BS>::PLX * ColorSweep<T, BS>::NW * ZG;
 }
@@ -273,8 +286,12 @@ __device__ __forceinline__ float ldval(const T *p) {
 // trigger stands at the end of a CTA: at its start, the next pass's CTAs took places on the
 // SMs early and unevenly (216 blocks: 13.4 -> 16.9 us; at the end 11.2 us).
 template <typename T, int BS, int FK, int ZG>
-__global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, ColorSweep<T, BS>::NT *ZG <= 256 ? 2 : 1)
-    kSweepColor(ColorArgs a) {
+constexpr int sweepCtas() {  // resident CTAs to leave registers for
+  return facesOnly<T, FK>() && BS == 32 ? 3 : ColorSweep<T, BS>::NT * ZG <= 256 ? 2 : 1;
+}
+
+template <typename T, int BS, int FK, int ZG>
+__global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK, ZG>()) kSweepColor(ColorArgs a) {
   using C = ColorSweep<T, BS>;
   using V4 = typename Vec4T<T>::V;
   constexpr int RS = C::RS, PL = C::PL, PLX = C::PLX, CZ = C::CZ, NCH = C::NCH;
@@ -314,7 +331,7 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, ColorSweep<T, BS>::
     const void *src[NCH];
     uint32_t b[NCH];
     auto prepare = [&](int k) {
-      const bool has = tid < C::NCC && tileCopy<T, BS>(k, tid, nbs, a, t, d[k], src[k], b[k]);
+      const bool has = tid < C::NCC && tileCopy<T, BS, FK>(k, tid, nbs, a, t, d[k], src[k], b[k]);
       if (!has) b[k] = 0;
       const uint32_t tot = __reduce_add_sync(0xffffffffu, b[k]);
       if (tid == 0) mbarExpectTx(&bar[k], tot);
@@ -526,7 +543,7 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, ColorSweep<T, BS>::
     // FP32 ring costs 26 wavefronts of shared memory a plane and warp where this takes 8 to
     // 11, and a barrier and a round trip per plane.  FP16 to FP32 is exact, so the window's
     // values are the ring's.  Measured (10 iterations): Jacobi on 514 M voxels 8.80 -> 6.12
-    // ms, MCF on 102 M voxels 2.73 -> 2.51 ms.  uint16 keeps the ring, which converts a
+    // ms (two CTAs an SM), MCF on 102 M voxels 2.73 -> 2.51 ms.  uint16 keeps the ring, which converts a
     // value once and a half (three times here) on the slower integer-to-float pipe.
     //
     // The thread's rows y-1, y, y+1 of plane p at (byte offset in shared memory) rowX + p *
@@ -589,7 +606,27 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, ColorSweep<T, BS>::
         r.ep = lds2(ep.at + p * ep.step);
       }
     };
+    uint2 zOut[2];  // facesOnly: the strip's voxels of planes -1 and BS, from the blocks below and above
+    if constexpr (facesOnly<T, FK>()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass wrote them
+#pragma unroll
+      for (int zi = 0; zi < 2; zi++) {
+        const int s = nbs[zi * 18 + 4];
+        if (s >= 0)
+          zOut[zi] = __ldcg(reinterpret_cast<const uint2 *>((const T *)a.payload + (int64_t)s * C::VPB +
+                                                            ((zi ? 0 : BS - 1) * BS + ty) * BS + tx));
+        else if (s == -1) zOut[zi] = lds8(offOf(t.er));
+      }
+    }
     auto fetchOut = [&](int p, Raw &r) {  // z-halo plane -1 or BS; the stencils read no edge of its rows y-1, y+1
+      if constexpr (facesOnly<T, FK>()) {  // and the 7-point form only the strip itself
+        const int zi = p < 0 ? 0 : 1, pc = zi ? BS - 1 : 0;
+        need(pc);
+        r.c = nbs[zi * 18 + 4] == -2 ? lds8(offOf(t.blk + (pc * BS + ty) * BS + tx)) : zOut[zi];
+        r.m = r.p = r.c;
+        r.em = r.ec = r.ep = 0;
+        return;
+      }
       const int zi = p < 0 ? 0 : 1, dzb = zi ? 1 : -1, pc = zi ? BS - 1 : 0;
       need(pc);
       auto row = [&](int y) -> uint2 {

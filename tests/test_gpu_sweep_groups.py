@@ -26,7 +26,8 @@ def _field(rng, n, vox, storage):
 # blocks a pass: 8 and 152 (four groups on 16^3 blocks, two on 32^3), 343 (two), 729 (one)
 CASES = [(16, 4, "F32", MCF8), (16, 4, "U16", MCF8), (16, 4, "F16", JAC8), (16, 4, "U16", LAPL8),
          (16, 14, "F32", MCF8), (16, 14, "U16", MCF8), (16, 18, "F32", MCF8), (16, 18, "F16", MCF8),
-         (16, 14, "F32", JAC8), (32, 4, "F16", MCF8), (32, 4, "F32", MCF8), (32, 11, "U16", MCF8), (32, 11, "F32", MCF8)]
+         (16, 14, "F32", JAC8), (32, 4, "F16", MCF8), (32, 4, "F16", JAC8), (32, 4, "F32", MCF8),
+         (32, 11, "U16", MCF8), (32, 11, "F32", MCF8)]
 
 
 @pytest.mark.parametrize("bsx,nb,storage,lapl", CASES)
