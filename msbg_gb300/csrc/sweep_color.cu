@@ -15,7 +15,7 @@
 // data into its private 2-slot ring of FP32 halo'd rows, so after the staging the
 // warps never wait for each other: only __syncwarp orders a warp's ring.  Results go straight to global
 // memory; the block is in shared memory before its first store, so the update
-// is in place.  FP16 channels skip the ring in all but the generic form: their threads
+// is in place.  FP16 and FP32 channels skip the ring in all but the generic form: their threads
 // read rows from the staged data (directRows).
 //
 // Halo traffic.  The block payload is x-fastest (src/sbg.h:1816-1820), so the
@@ -155,9 +155,9 @@ struct ColorArgs {
   SweepParams p;
 };
 
-// Stencil forms that read FP16 rows straight from the staged tile (see kSweepColor).
+// Stencil forms that read rows straight from the staged tile (see kSweepColor).
 template <typename T, int FK>
-constexpr bool directRows() { return std::is_same<T, __half>::value && FK != 0; }
+constexpr bool directRows() { return !std::is_same<T, uint16_t>::value && FK != 0; }
 
 // The direct 7-point form: a thread needs its own four voxels of the planes z=-1 and z=BS, which
 // it reads from global memory, and no corner.  Without those pieces (4.9 KB) three CTAs of a
@@ -165,7 +165,7 @@ constexpr bool directRows() { return std::is_same<T, __half>::value && FK != 0; 
 // for the direct MCF form (80 registers, planes from global memory) was slower on 102 M voxels,
 // 2.51 -> 2.66 ms.
 template <typename T, int FK>
-constexpr bool facesOnly() { return directRows<T, FK>() && (FK & ~FK_CLAMP) == K_JACOBI; }
+constexpr bool facesOnly() { return std::is_same<T, __half>::value && (FK & ~FK_CLAMP) == K_JACOBI; }
 
 // Copy slot c of chunk k (planes k*CZ .. k*CZ+CZ-1) of a block's tile: fills
 // (dst, src, bytes) and returns true when the piece exists (its source block is a
@@ -537,14 +537,15 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
   using Interior = std::integral_constant<int, 0>;
 
   if constexpr (directRows<T, FK>()) {
-    // FP16 rows are narrow enough to be read where they are staged: a thread reads its own
-    // strip of rows y-1, y, y+1 as one 8-byte load each, widens them, and takes the values
-    // beside the strip from the neighbouring lanes (block sides: one 2-byte load more).  The
-    // FP32 ring costs 26 wavefronts of shared memory a plane and warp where this takes 8 to
-    // 11, and a barrier and a round trip per plane.  FP16 to FP32 is exact, so the window's
-    // values are the ring's.  Measured (10 iterations): Jacobi on 514 M voxels 8.80 -> 6.12
-    // ms (two CTAs an SM), MCF on 102 M voxels 2.73 -> 2.51 ms.  uint16 keeps the ring, which converts a
-    // value once and a half (three times here) on the slower integer-to-float pipe.
+    // Rows are read where they are staged: a thread reads its own strip of rows y-1, y, y+1 as
+    // one 8- or 16-byte load each, widens FP16, and takes the values beside the strip from the
+    // neighbouring lanes (block sides: one narrow load more).  The FP32 ring costs 26 wavefronts
+    // of shared memory a plane and warp where FP16 takes 8 to 11 here and FP32 14 to 17, and a
+    // barrier and a round trip per plane.  FP16 to FP32 is exact, so the window's values are the
+    // ring's.  Measured: FP16, 10 iterations, Jacobi on 514 M voxels 8.80 -> 6.12 ms (two CTAs
+    // an SM), MCF on 102 M voxels 2.73 -> 2.51 ms; FP32, 20 iterations of the exact MCF on 14 M
+    // voxels 2.88 -> 2.75 ms.  uint16 keeps the ring, which converts a value once and a half
+    // (three times here) on the slower integer-to-float pipe.
     //
     // The thread's rows y-1, y, y+1 of plane p at (byte offset in shared memory) rowX + p *
     // stepX, and the value beyond the block's side, in the lanes that need one, at edgeX.
@@ -581,55 +582,60 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
     const Walk wm = rowSrc(ty - 1), wp = rowSrc(ty + 1), ec = edgeSrc(ty);
     const Walk em = kCorners ? edgeSrc(ty - 1) : Walk{0, 0}, ep = kCorners ? edgeSrc(ty + 1) : Walk{0, 0};
     const uint32_t rowC = offOf(t.blk + ty * BS + tx);
-    auto lds8 = [&](uint32_t off) {
-      uint2 v;
-      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(tb + off));
+    using E = std::conditional_t<sizeof(T) == 4, float, uint16_t>;  // an edge value's bits
+    auto ldsRow = [&](uint32_t off) {
+      V4 v;
+      if constexpr (sizeof(T) == 4)
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(tb + off));
+      else
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(tb + off));
       return v;
     };
-    auto lds2 = [&](uint32_t off) {
-      uint16_t v;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(tb + off));
+    auto ldsEdge = [&](uint32_t off) {
+      E v;
+      if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(tb + off));
+      else asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(tb + off));
       return v;
     };
     struct Raw {
-      uint2 m, c, p;
-      uint16_t em, ec, ep;
+      V4 m, c, p;
+      E em, ec, ep;
     };
     auto fetchIn = [&](int p, Raw &r) {  // plane 0 .. BS-1
       need(p);
-      r.m = lds8(wm.at + p * wm.step);
-      r.c = lds8(rowC + p * (uint32_t)(BS * BS * sizeof(T)));
-      r.p = lds8(wp.at + p * wp.step);
-      r.ec = lds2(ec.at + p * ec.step);
+      r.m = ldsRow(wm.at + p * wm.step);
+      r.c = ldsRow(rowC + p * (uint32_t)(BS * BS * sizeof(T)));
+      r.p = ldsRow(wp.at + p * wp.step);
+      r.ec = ldsEdge(ec.at + p * ec.step);
       if constexpr (kCorners) {
-        r.em = lds2(em.at + p * em.step);
-        r.ep = lds2(ep.at + p * ep.step);
+        r.em = ldsEdge(em.at + p * em.step);
+        r.ep = ldsEdge(ep.at + p * ep.step);
       }
     };
-    uint2 zOut[2];  // facesOnly: the strip's voxels of planes -1 and BS, from the blocks below and above
+    V4 zOut[2];  // facesOnly: the strip's voxels of planes -1 and BS, from the blocks below and above
     if constexpr (facesOnly<T, FK>()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass wrote them
 #pragma unroll
       for (int zi = 0; zi < 2; zi++) {
         const int s = nbs[zi * 18 + 4];
         if (s >= 0)
-          zOut[zi] = __ldcg(reinterpret_cast<const uint2 *>((const T *)a.payload + (int64_t)s * C::VPB +
+          zOut[zi] = __ldcg(reinterpret_cast<const V4 *>((const T *)a.payload + (int64_t)s * C::VPB +
                                                             ((zi ? 0 : BS - 1) * BS + ty) * BS + tx));
-        else if (s == -1) zOut[zi] = lds8(offOf(t.er));
+        else if (s == -1) zOut[zi] = ldsRow(offOf(t.er));
       }
     }
     auto fetchOut = [&](int p, Raw &r) {  // z-halo plane -1 or BS; the stencils read no edge of its rows y-1, y+1
       if constexpr (facesOnly<T, FK>()) {  // and the 7-point form only the strip itself
         const int zi = p < 0 ? 0 : 1, pc = zi ? BS - 1 : 0;
         need(pc);
-        r.c = nbs[zi * 18 + 4] == -2 ? lds8(offOf(t.blk + (pc * BS + ty) * BS + tx)) : zOut[zi];
+        r.c = nbs[zi * 18 + 4] == -2 ? ldsRow(offOf(t.blk + (pc * BS + ty) * BS + tx)) : zOut[zi];
         r.m = r.p = r.c;
         r.em = r.ec = r.ep = 0;
         return;
       }
       const int zi = p < 0 ? 0 : 1, dzb = zi ? 1 : -1, pc = zi ? BS - 1 : 0;
       need(pc);
-      auto row = [&](int y) -> uint2 {
+      auto row = [&](int y) -> V4 {
         const T *q;
         if (y >= 0 && y < BS) {
           const int s = nbs[(dzb + 1) * 9 + 4];
@@ -638,29 +644,36 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
           const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1, s = nbs[(dzb + 1) * 9 + (dy + 1) * 3 + 1];
           q = s >= 0 ? t.zh[zi][dy < 0 ? 2 : 3] + tx : s == -1 ? t.er : t.blk + (pc * BS + yc) * BS + tx;
         }
-        return lds8(offOf(q));
+        return ldsRow(offOf(q));
       };
       r.m = row(ty - 1);
       r.c = row(ty);
       r.p = row(ty + 1);
       const int side = atFirst ? 0 : 1, s = nbs[(dzb + 1) * 9 + 3 + (side ? 2 : 0)];
-      r.ec = lds2(offOf(s >= 0 ? t.zh[zi][side] + ty : s == -1 ? t.er : t.blk + (pc * BS + ty) * BS + (side ? BS - 1 : 0)));
+      r.ec = ldsEdge(offOf(s >= 0 ? t.zh[zi][side] + ty : s == -1 ? t.er : t.blk + (pc * BS + ty) * BS + (side ? BS - 1 : 0)));
       r.em = r.ep = 0;
     };
-    auto half4 = [](const uint2 &v, float o[4]) {
-      const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-      const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-      o[0] = lo.x; o[1] = lo.y; o[2] = hi.x; o[3] = hi.y;
+    auto unpackRow = [](const V4 &v, float o[4]) {
+      if constexpr (sizeof(T) == 4) {
+        o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+      } else {
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+        const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+        o[0] = lo.x; o[1] = lo.y; o[2] = hi.x; o[3] = hi.y;
+      }
     };
-    auto half1 = [](uint16_t v) { return __half2float(__ushort_as_half(v)); };
+    auto edgeVal = [](E v) {
+      if constexpr (sizeof(T) == 4) return v;
+      else return __half2float(__ushort_as_half(v));
+    };
     auto plane = [&](const Raw &r, PW &W) {
       StripRows s;
-      half4(r.m, s.m);
-      half4(r.c, s.c);
-      half4(r.p, s.p);
-      s.ec = half1(r.ec);
+      unpackRow(r.m, s.m);
+      unpackRow(r.c, s.c);
+      unpackRow(r.p, s.p);
+      s.ec = edgeVal(r.ec);
       s.em = s.ep = 0.0f;
-      if constexpr (kCorners) { s.em = half1(r.em); s.ep = half1(r.ep); }
+      if constexpr (kCorners) { s.em = edgeVal(r.em); s.ep = edgeVal(r.ep); }
       planeOf(s, atFirst, atLast, W);
     };
     auto fetch = [&](int p, Raw &r) {
