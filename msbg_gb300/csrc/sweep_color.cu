@@ -10,13 +10,10 @@
 // first chunk has landed.  Each thread owns a 4-voxel x-strip of every plane and
 // marches through the block in z with a register window of three planes (rows
 // y-1..y+1, columns x-1..x+4 of planes z-1, z, z+1; the three windows rotate
-// roles, so no register moves).  Each warp owns 4 rows (32^3) of every plane and
-// converts the rows it needs (its own and one on each side) from the staged raw
-// data into its private 2-slot ring of FP32 halo'd rows, so after the staging the
-// warps never wait for each other: only __syncwarp orders a warp's ring.  Results go straight to global
-// memory; the block is in shared memory before its first store, so the update
-// is in place.  FP16 and FP32 channels skip the ring in all but the generic form: their threads
-// read rows from the staged data (directRows).
+// roles, so no register moves).  It reads its strips straight from the staged
+// data, so after the staging the warps never wait for each other.  Results go
+// straight to global memory; the block is in shared memory before its first
+// store, so the update is in place.
 //
 // Halo traffic.  The block payload is x-fastest (src/sbg.h:1816-1820), so the
 // y- and z-neighbour rows/planes are contiguous but an x-neighbour column is one
@@ -42,17 +39,6 @@ template <> struct Vec4T<__half> { using V = uint2; };
 template <> struct Vec4T<uint16_t> { using V = uint2; };
 
 template <typename T>
-__device__ __forceinline__ void unpack4(const typename Vec4T<T>::V &v, float o[4]) {
-  if constexpr (sizeof(T) == 4) {
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  } else {
-    const T *e = reinterpret_cast<const T *>(&v);
-#pragma unroll
-    for (int k = 0; k < 4; k++) o[k] = Store<T>::load(e + k);
-  }
-}
-
-template <typename T>
 __device__ __forceinline__ typename Vec4T<T>::V pack4(const float o[4]) {
   typename Vec4T<T>::V v;
   if constexpr (sizeof(T) == 4) {
@@ -75,17 +61,6 @@ template <typename T, int BS>
 struct ColorSweep {
   static constexpr int NT = BS * BS / 4;     // threads: one 4-voxel x-strip of every plane each
   static constexpr int SPR = BS / 4;         // strips per row
-  static constexpr int RPW = 32 / SPR;       // rows per warp
-  static constexpr int NW = NT / 32;         // warps
-  static constexpr int RS = BS + 8;          // ring row stride (floats); x in [-1,BS] at col x+4
-  static constexpr int WR = RPW + 2;         // rows of a warp's ring plane (its rows +-1)
-  static constexpr int PL = WR * RS;         // floats per warp ring plane (2 slots per warp)
-  static constexpr int PLX = PL + 4;         // slot stride: a 4-float tail takes the fills of idle lanes
-  static constexpr int NG = WR * SPR;        // 4-value groups of a warp ring plane
-  static constexpr int NGP = (NG + 31) / 32; // groups per lane
-  static constexpr int NXH = 2 * WR;         // x-halo values of a warp ring plane
-  static constexpr int NHALO = 4 * BS + 4;   // halo elements of a plane (2 cols, 2 rows, 4 corners)
-  static constexpr int NH = NHALO <= NT ? 1 : (NHALO + NT - 1) / NT;
   static constexpr int64_t VPB = (int64_t)BS * BS * BS;
   static constexpr int FACE = BS * BS;       // per x-face
   static constexpr int CORN = BS;            // per corner column
@@ -101,7 +76,7 @@ struct RawTile {
   T xf[2][BS * BS];      // column x=-1 (0) and x=BS (1), [z][y]
   T yr[2][BS * BS];      // row y=-1 (0) and y=BS (1), [z][x]
   alignas(16) T er[16];  // the empty value (source of every fill from an empty block)
-  // from here on not staged by the direct 7-point form (facesOnly)
+  // from here on not staged by the fast 7-point form (facesOnly)
   T zpl[2][BS * BS];     // plane z=-1 (0) and z=BS (1), [y][x]
   T cn[4][BS];           // corner columns (x=-1|BS, y=-1|BS), k = (dx>0) + 2*(dy>0), [z]
   T zh[2][4][BS];        // planes -1 / BS: x=-1 row, x=BS row (over y), y=-1 row, y=BS row (over x)
@@ -155,17 +130,13 @@ struct ColorArgs {
   SweepParams p;
 };
 
-// Stencil forms that read rows straight from the staged tile (see kSweepColor).
-template <typename T, int FK>
-constexpr bool directRows() { return !std::is_same<T, uint16_t>::value && FK != 0; }
-
-// The direct 7-point form: a thread needs its own four voxels of the planes z=-1 and z=BS, which
+// The fast 7-point form: a thread needs its own four voxels of the planes z=-1 and z=BS, which
 // it reads from global memory, and no corner.  Without those pieces (4.9 KB) three CTAs of a
-// 32^3 block share an SM (72 registers): 514 M voxels, 10 iterations, 6.12 -> 4.92 ms.  The same
-// for the direct MCF form (80 registers, planes from global memory) was slower on 102 M voxels,
-// 2.51 -> 2.66 ms.
+// 32^3 block share an SM (72 registers): FP16, 514 M voxels, 10 iterations, 6.12 -> 4.92 ms.
+// The same for MCF (80 registers, planes from global memory) was slower on 102 M voxels, 2.51 ->
+// 2.66 ms.
 template <typename T, int FK>
-constexpr bool facesOnly() { return std::is_same<T, __half>::value && (FK & ~FK_CLAMP) == K_JACOBI; }
+constexpr bool facesOnly() { return sizeof(T) == 2 && (FK & ~FK_CLAMP) == K_JACOBI; }
 
 // Copy slot c of chunk k (planes k*CZ .. k*CZ+CZ-1) of a block's tile: fills
 // (dst, src, bytes) and returns true when the piece exists (its source block is a
@@ -257,17 +228,11 @@ constexpr size_t rawTileBytes() {
   return (sizeof(RawTile<T, BS>) + 15) & ~size_t(15);
 }
 
-template <typename T, int BS, int FK, int ZG>
+template <typename T, int BS, int FK>
 constexpr size_t colorSmemBytes() {
   using Tile = RawTile<T, BS>;
   if (facesOnly<T, FK>()) return offsetof(Tile, zpl);
-  if (directRows<T, FK>()) return rawTileBytes<T, BS>();
-  return rawTileBytes<T, BS>() + 2 * sizeof(float) * ColorSweep<T, BS>::PLX * ColorSweep<T, BS>::NW * ZG;
-}
-
-template <typename T>
-__device__ __forceinline__ float ldval(const T *p) {
-  if constexpr (sizeof(T) == 4) return *p; else return Store<T>::load(p);
+  return rawTileBytes<T, BS>();
 }
 
 // FK: the stencil, fixed at compile time.  0 = any kind in the reference's
@@ -281,20 +246,22 @@ __device__ __forceinline__ float ldval(const T *p) {
 //
 // The passes of a call are launched with programmatic serialization: a pass's CTAs look up
 // their blocks and neighbours and prepare their copies while the previous pass drains, and
-// wait for its writes (griddepcontrol.wait) before the first copy.  Only warp 0 waits: what
-// the other warps read arrives through its copies, and what they write comes after.  The
+// wait for its writes (griddepcontrol.wait) before the first copy.  Only warp 0 waits (all warps
+// where facesOnly reads planes directly): what the other warps read arrives through its copies,
+// and what they write comes after.  The
 // trigger stands at the end of a CTA: at its start, the next pass's CTAs took places on the
 // SMs early and unevenly (216 blocks: 13.4 -> 16.9 us; at the end 11.2 us).
 template <typename T, int BS, int FK, int ZG>
 constexpr int sweepCtas() {  // resident CTAs to leave registers for
-  return facesOnly<T, FK>() && BS == 32 ? 3 : ColorSweep<T, BS>::NT * ZG <= 256 ? 2 : 1;
+  constexpr int nt = ColorSweep<T, BS>::NT * ZG;
+  return facesOnly<T, FK>() && BS == 32 ? 3 : nt <= 256 ? 512 / nt : 1;
 }
 
 template <typename T, int BS, int FK, int ZG>
 __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK, ZG>()) kSweepColor(ColorArgs a) {
   using C = ColorSweep<T, BS>;
   using V4 = typename Vec4T<T>::V;
-  constexpr int RS = C::RS, PL = C::PL, PLX = C::PLX, CZ = C::CZ, NCH = C::NCH;
+  constexpr int CZ = C::CZ, NCH = C::NCH;
   constexpr int PZ = BS / ZG;  // planes of a z-group
   extern __shared__ __align__(128) unsigned char dynSmem[];
   RawTile<T, BS> &t = *reinterpret_cast<RawTile<T, BS> *>(dynSmem);
@@ -350,66 +317,11 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
   }
 
   const int ownSlot = nbs[13];
-  const int lane = tid & 31, zg = tid / C::NT, gt = tid % C::NT;
-  const int warp = gt >> 5;                              // warp within the z-group
+  const int zg = tid / C::NT, gt = tid % C::NT;
   const int zFirst = zg * PZ;                            // first plane of the z-group
   const int ty = gt / C::SPR, tx = (gt % C::SPR) * 4;    // this thread's strip
-  const int y0w = warp * C::RPW;                          // first row of this warp
-  const int tyl = ty - y0w;                               // row inside the warp
-  float *wring = reinterpret_cast<float *>(dynSmem + rawTileBytes<T, BS>()) + (tid >> 5) * 2 * PLX;
-  float emptyF;
-  {
-    T e;
-    if constexpr (sizeof(T) == 4) e = a.emptyValue; else Store<T>::storeRNE(&e, a.emptyValue);
-    if constexpr (sizeof(T) == 4) emptyF = e; else emptyF = Store<T>::load(&e);
-  }
-
-  // ---- per-lane fill sources for the interior planes 0..BS-1 ------------------
-  // Quad groups: ring row rr (y = y0w-1+rr), x = 4j..4j+3; source = base + p*stride.
-  // Every lane gets a source for each of its groups: an empty block (and a lane
-  // without a k-th group) reads the empty row with stride 0; an idle lane writes to
-  // the slot's 4-float tail.  The fill then has no branches.
-  const T *gSrc[C::NGP];
-  int gStride[C::NGP], gDst[C::NGP];
-#pragma unroll
-  for (int k = 0; k < C::NGP; k++) {
-    const int g = lane + 32 * k;
-    const int rr = g / C::SPR, j = g % C::SPR, y = y0w - 1 + rr, x = 4 * j;
-    gDst[k] = g < C::NG ? rr * RS + x + 4 : PL;
-    gSrc[k] = t.er;
-    gStride[k] = 0;
-    if (g < C::NG) {
-      if (y >= 0 && y < BS) {
-        gSrc[k] = t.blk + y * BS + x; gStride[k] = BS * BS;
-      } else {
-        const int side = y < 0 ? 0 : 1;
-        const int s = nbs[9 + (side ? 2 : 0) * 3 + 1];
-        if (s >= 0) { gSrc[k] = t.yr[side] + x; gStride[k] = BS; }
-        else if (s != -1) { gSrc[k] = t.blk + (side ? BS - 1 : 0) * BS + x; gStride[k] = BS * BS; }  // Neumann
-      }
-    }
-  }
-  // x-halo values: side = lane / WR (x=-1 | x=BS), ring row rr = lane % WR
-  const T *hSrc = t.er;
-  int hStride = 0, hDst = PL;
-  if (lane < C::NXH) {
-    const int side = lane / C::WR, rr = lane % C::WR, y = y0w - 1 + rr;
-    const int dx = side ? 1 : -1, xc = side ? BS - 1 : 0;
-    hDst = rr * RS + (side ? BS + 4 : 3);
-    if (y >= 0 && y < BS) {
-      const int s = nbs[9 + 3 + (dx + 1)];
-      if (s >= 0) { hSrc = t.xf[side] + y; hStride = BS; }
-      else if (s != -1) { hSrc = t.blk + y * BS + xc; hStride = BS * BS; }
-    } else {  // corner column of the diagonal neighbour
-      const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1;
-      const int s = nbs[9 + (dy + 1) * 3 + (dx + 1)];
-      if (s >= 0) { hSrc = t.cn[(dx > 0 ? 1 : 0) + 2 * (dy > 0 ? 1 : 0)]; hStride = 1; }
-      else if (s != -1) { hSrc = t.blk + yc * BS + xc; hStride = BS * BS; }
-    }
-  }
-
-  // planes are consumed in increasing order (fillZ(-1) needs chunk 0, fillZ(BS)
-  // comes after plane BS-1), so one counter of the planes known to have landed
+  // planes are consumed in increasing order (plane -1 needs chunk 0, plane BS comes after
+  // plane BS-1), so one counter of the planes known to have landed
   // replaces per-chunk flags
   int readyPlanes = 0;
   bool timedOut = false;
@@ -420,73 +332,10 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
     }
   };
 
-  // ---- interior plane p (0..BS-1) -> this warp's ring slot, in two halves so
-  // that the shared-memory reads of plane p overlap the previous plane's update ----
-  V4 rawG[C::NGP];
-  T rawH;
-  auto loadRaw = [&](int p) {
-    need(p);
-#pragma unroll
-    for (int k = 0; k < C::NGP; k++) rawG[k] = *reinterpret_cast<const V4 *>(gSrc[k] + p * gStride[k]);
-    rawH = hSrc[p * hStride];
-  };
-  auto storeRaw = [&](float *pl) {
-#pragma unroll
-    for (int k = 0; k < C::NGP; k++) {
-      float q[4];
-      unpack4<T>(rawG[k], q);
-      *reinterpret_cast<float4 *>(pl + gDst[k]) = make_float4(q[0], q[1], q[2], q[3]);
-    }
-    pl[hDst] = ldval<T>(&rawH);
-  };
-  auto fillInterior = [&](int p, float *pl) {
-    loadRaw(p);
-    storeRaw(pl);
-  };
-
-  // ---- z-halo plane p = -1 or BS -> this warp's ring slot (twice per block) ----
-  auto fillZ = [&](int p, float *pl) {
-    const int zi = p < 0 ? 0 : 1;
-    need(zi ? BS - 1 : 0);
-    const int dzb = zi ? 1 : -1;
-    const int pc = zi ? BS - 1 : 0;  // Neumann clamp inside the own block
-    for (int g = lane; g < C::NG; g += 32) {
-      const int rr = g / C::SPR, j = g % C::SPR, y = y0w - 1 + rr, x = 4 * j;
-      float q[4] = {emptyF, emptyF, emptyF, emptyF};
-      if (y >= 0 && y < BS) {
-        const int s = nbs[(dzb + 1) * 9 + 4];
-        if (s >= 0) unpack4<T>(*reinterpret_cast<const V4 *>(t.zpl[zi] + y * BS + x), q);
-        else if (s == -2) unpack4<T>(*reinterpret_cast<const V4 *>(t.blk + (pc * BS + y) * BS + x), q);
-      } else {
-        const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1;
-        const int s = nbs[(dzb + 1) * 9 + (dy + 1) * 3 + 1];
-        if (s >= 0) unpack4<T>(*reinterpret_cast<const V4 *>(t.zh[zi][dy < 0 ? 2 : 3] + x), q);
-        else if (s == -2) unpack4<T>(*reinterpret_cast<const V4 *>(t.blk + (pc * BS + yc) * BS + x), q);
-      }
-      *reinterpret_cast<float4 *>(pl + rr * RS + x + 4) = make_float4(q[0], q[1], q[2], q[3]);
-    }
-    if (lane < C::NXH) {
-      const int side = lane / C::WR, rr = lane % C::WR, y = y0w - 1 + rr;
-      const int dx = side ? 1 : -1, xc = side ? BS - 1 : 0;
-      float f = 0.0f;  // x-halo corners of a z-halo plane are read by no stencil
-      if (y >= 0 && y < BS) {
-        const int s = nbs[(dzb + 1) * 9 + 3 + (dx + 1)];
-        if (s >= 0) f = ldval<T>(t.zh[zi][side] + y);
-        else if (s == -1) f = emptyF;
-        else f = ldval<T>(t.blk + (pc * BS + y) * BS + xc);
-      }
-      pl[rr * RS + (side ? BS + 4 : 3)] = f;
-    }
-  };
-
-  // ---- warp ring slot -> this thread's plane (rows y-1..y+1, x-1..x+4) ----
   constexpr int FKK = FK & ~FK_CLAMP;
   using PW = std::conditional_t<
       FKK == K_MCF, PlaneMcf,
       std::conditional_t<FKK == K_JACOBI, PlaneJac, std::conditional_t<FKK == (K_MCF | FK_EXACT), PlaneMcfX, PlaneRaw>>>;
-  const int winOff = tyl * RS + tx + 3;
-  auto window = [&](const float *pl, PW &w) { loadPlane<RS>(pl + winOff, w); };
-
   T *outp = (T *)a.payload + (int64_t)ownSlot * C::VPB + ty * BS + tx;
   // x-face / corner cache entries this thread maintains (x = 0 or BS-1 strips)
   const bool faceThread = tx == 0 || tx == BS - 4;
@@ -515,284 +364,182 @@ __global__ void __launch_bounds__(ColorSweep<T, BS>::NT *ZG, sweepCtas<T, BS, FK
     if (faceThread) facep[z * BS] = v;
     if (cornThread) cornp[z] = v;
   };
-  // One plane.  On entry A, B, C hold planes z-1, z, z+1 and, for an interior
-  // plane z+2, its raw values are in registers.  Plane z+2 is staged into the
-  // warp's ring slot (z & 1), which held plane z, last read before the previous
-  // step's __syncwarp; the raw values of plane z+3 are read; on exit A holds
-  // plane z+2.  KIND: 0 = planes z+2 and z+3 are interior planes, 3 = only plane
-  // z+2 is, 1 = plane z+2 is the z-halo plane BS, 2 = there is no plane z+2.
-  auto step = [&](auto kind, int z, PW &A, PW &B, PW &Cw) {
-    constexpr int KIND = decltype(kind)::value;
-    float *slot = wring + (z & 1) * PLX;
-    if constexpr (KIND == 0 || KIND == 3) {
-      storeRaw(slot);
-      if constexpr (KIND == 0) loadRaw(z + 3);
-    } else if constexpr (KIND == 1) {
-      fillZ(BS, slot);
-    }
-    __syncwarp();
-    emit(z, A, B, Cw);
-    if constexpr (KIND != 2) window(slot, A);
+  // Rows are read where they are staged: a thread reads its own strip of rows y-1, y, y+1 as
+  // one 8- or 16-byte load each, widens them (exactly), and takes the values beside the strip
+  // from the neighbouring lanes (block sides: one narrow load more).  A ring of FP32 rows in
+  // shared memory, converted once per warp, costs 26 wavefronts a plane and warp where FP16
+  // takes 8 to 11 here and FP32 14 to 17, and a barrier and a round trip per plane.  The march
+  // is unrolled by three, which saves the moves of the rotating windows.  Measured against the
+  // ring, us a pass: FP16 32^3 blocks, 512 a pass, exact MCF 66.9 -> 52.2, fast MCF 41.6 ->
+  // 37.9, Jacobi 32.1 -> 22.6; 16^3 blocks, 1000 a pass, exact MCF (FP32) 22.8 -> 18.8, fast
+  // MCF 22.5 -> 14.4, Jacobi 15.0 -> 10.8; 64 blocks 6.2 -> 5.3, 5.6 -> 4.7, 4.9 -> 4.2.
+  //
+  // The thread's rows y-1, y, y+1 of plane p at (byte offset in shared memory) rowX + p *
+  // stepX, and the value beyond the block's side, in the lanes that need one, at edgeX.
+  // Offsets rather than pointers: a source is a 32-bit word, a step another.
+  const bool atFirst = tx == 0, atLast = tx == BS - 4;
+  const uint32_t tb = smemAddr(&t);
+  auto offOf = [&](const void *q) { return smemAddr(q) - tb; };
+  struct Walk {
+    uint32_t at, step;
   };
-  using Interior = std::integral_constant<int, 0>;
-
-  if constexpr (directRows<T, FK>()) {
-    // Rows are read where they are staged: a thread reads its own strip of rows y-1, y, y+1 as
-    // one 8- or 16-byte load each, widens FP16, and takes the values beside the strip from the
-    // neighbouring lanes (block sides: one narrow load more).  The FP32 ring costs 26 wavefronts
-    // of shared memory a plane and warp where FP16 takes 8 to 11 here and FP32 14 to 17, and a
-    // barrier and a round trip per plane.  FP16 to FP32 is exact, so the window's values are the
-    // ring's.  Measured: FP16, 10 iterations, Jacobi on 514 M voxels 8.80 -> 6.12 ms (two CTAs
-    // an SM), MCF on 102 M voxels 2.73 -> 2.51 ms; FP32, 20 iterations of the exact MCF on 14 M
-    // voxels 2.88 -> 2.75 ms.  uint16 keeps the ring, which converts a value once and a half
-    // (three times here) on the slower integer-to-float pipe.
-    //
-    // The thread's rows y-1, y, y+1 of plane p at (byte offset in shared memory) rowX + p *
-    // stepX, and the value beyond the block's side, in the lanes that need one, at edgeX.
-    // Offsets rather than pointers: a source is a 32-bit word, a step another.
-    const bool atFirst = tx == 0, atLast = tx == BS - 4;
-    const uint32_t tb = smemAddr(&t);
-    auto offOf = [&](const void *q) { return smemAddr(q) - tb; };
-    struct Walk {
-      uint32_t at, step;
-    };
-    // row y of the own block, its y-neighbour, the empty row, or (domain boundary) the nearest own row
-    auto rowSrc = [&](int y) -> Walk {
-      if (y >= 0 && y < BS) return {offOf(t.blk + y * BS + tx), BS * BS * sizeof(T)};
-      const int side = y < 0 ? 0 : 1, s = nbs[9 + (side ? 2 : 0) * 3 + 1];
-      if (s >= 0) return {offOf(t.yr[side] + tx), BS * sizeof(T)};
+  // row y of the own block, its y-neighbour, the empty row, or (domain boundary) the nearest own row
+  auto rowSrc = [&](int y) -> Walk {
+    if (y >= 0 && y < BS) return {offOf(t.blk + y * BS + tx), BS * BS * sizeof(T)};
+    const int side = y < 0 ? 0 : 1, s = nbs[9 + (side ? 2 : 0) * 3 + 1];
+    if (s >= 0) return {offOf(t.yr[side] + tx), BS * sizeof(T)};
+    if (s == -1) return {offOf(t.er), 0u};
+    return {offOf(t.blk + (side ? BS - 1 : 0) * BS + tx), BS * BS * sizeof(T)};
+  };
+  auto edgeSrc = [&](int y) -> Walk {
+    if (!atFirst && !atLast) return {offOf(t.er), 0u};
+    const int side = atFirst ? 0 : 1, dx = side ? 1 : -1, xc = side ? BS - 1 : 0;
+    if (y >= 0 && y < BS) {
+      const int s = nbs[9 + 3 + (dx + 1)];
+      if (s >= 0) return {offOf(t.xf[side] + y), BS * sizeof(T)};
       if (s == -1) return {offOf(t.er), 0u};
-      return {offOf(t.blk + (side ? BS - 1 : 0) * BS + tx), BS * BS * sizeof(T)};
-    };
-    auto edgeSrc = [&](int y) -> Walk {
-      if (!atFirst && !atLast) return {offOf(t.er), 0u};
-      const int side = atFirst ? 0 : 1, dx = side ? 1 : -1, xc = side ? BS - 1 : 0;
-      if (y >= 0 && y < BS) {
-        const int s = nbs[9 + 3 + (dx + 1)];
-        if (s >= 0) return {offOf(t.xf[side] + y), BS * sizeof(T)};
-        if (s == -1) return {offOf(t.er), 0u};
-        return {offOf(t.blk + y * BS + xc), BS * BS * sizeof(T)};
-      }
-      const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1, s = nbs[9 + (dy + 1) * 3 + (dx + 1)];
-      if (s >= 0) return {offOf(t.cn[(dx > 0 ? 1 : 0) + 2 * (dy > 0 ? 1 : 0)]), (uint32_t)sizeof(T)};
-      if (s == -1) return {offOf(t.er), 0u};
-      return {offOf(t.blk + yc * BS + xc), BS * BS * sizeof(T)};
-    };
-    constexpr bool kCorners = FKK != K_JACOBI;  // the 7-point form reads no edge of rows y-1, y+1
-    const Walk wm = rowSrc(ty - 1), wp = rowSrc(ty + 1), ec = edgeSrc(ty);
-    const Walk em = kCorners ? edgeSrc(ty - 1) : Walk{0, 0}, ep = kCorners ? edgeSrc(ty + 1) : Walk{0, 0};
-    const uint32_t rowC = offOf(t.blk + ty * BS + tx);
-    using E = std::conditional_t<sizeof(T) == 4, float, uint16_t>;  // an edge value's bits
-    auto ldsRow = [&](uint32_t off) {
-      V4 v;
-      if constexpr (sizeof(T) == 4)
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(tb + off));
-      else
-        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(tb + off));
-      return v;
-    };
-    auto ldsEdge = [&](uint32_t off) {
-      E v;
-      if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(tb + off));
-      else asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(tb + off));
-      return v;
-    };
-    struct Raw {
-      V4 m, c, p;
-      E em, ec, ep;
-    };
-    auto fetchIn = [&](int p, Raw &r) {  // plane 0 .. BS-1
-      need(p);
-      r.m = ldsRow(wm.at + p * wm.step);
-      r.c = ldsRow(rowC + p * (uint32_t)(BS * BS * sizeof(T)));
-      r.p = ldsRow(wp.at + p * wp.step);
-      r.ec = ldsEdge(ec.at + p * ec.step);
-      if constexpr (kCorners) {
-        r.em = ldsEdge(em.at + p * em.step);
-        r.ep = ldsEdge(ep.at + p * ep.step);
-      }
-    };
-    V4 zOut[2];  // facesOnly: the strip's voxels of planes -1 and BS, from the blocks below and above
-    if constexpr (facesOnly<T, FK>()) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass wrote them
+      return {offOf(t.blk + y * BS + xc), BS * BS * sizeof(T)};
+    }
+    const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1, s = nbs[9 + (dy + 1) * 3 + (dx + 1)];
+    if (s >= 0) return {offOf(t.cn[(dx > 0 ? 1 : 0) + 2 * (dy > 0 ? 1 : 0)]), (uint32_t)sizeof(T)};
+    if (s == -1) return {offOf(t.er), 0u};
+    return {offOf(t.blk + yc * BS + xc), BS * BS * sizeof(T)};
+  };
+  constexpr bool kCorners = FKK != K_JACOBI;  // the 7-point form reads no edge of rows y-1, y+1
+  const Walk wm = rowSrc(ty - 1), wp = rowSrc(ty + 1), ec = edgeSrc(ty);
+  const Walk em = kCorners ? edgeSrc(ty - 1) : Walk{0, 0}, ep = kCorners ? edgeSrc(ty + 1) : Walk{0, 0};
+  const uint32_t rowC = offOf(t.blk + ty * BS + tx);
+  using E = std::conditional_t<sizeof(T) == 4, float, uint16_t>;  // an edge value's bits
+  auto ldsRow = [&](uint32_t off) {
+    V4 v;
+    if constexpr (sizeof(T) == 4)
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(tb + off));
+    else
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(tb + off));
+    return v;
+  };
+  auto ldsEdge = [&](uint32_t off) {
+    E v;
+    if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(tb + off));
+    else asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(tb + off));
+    return v;
+  };
+  struct Raw {
+    V4 m, c, p;
+    E em, ec, ep;
+  };
+  auto fetchIn = [&](int p, Raw &r) {  // plane 0 .. BS-1
+    need(p);
+    r.m = ldsRow(wm.at + p * wm.step);
+    r.c = ldsRow(rowC + p * (uint32_t)(BS * BS * sizeof(T)));
+    r.p = ldsRow(wp.at + p * wp.step);
+    r.ec = ldsEdge(ec.at + p * ec.step);
+    if constexpr (kCorners) {
+      r.em = ldsEdge(em.at + p * em.step);
+      r.ep = ldsEdge(ep.at + p * ep.step);
+    }
+  };
+  V4 zOut[2];  // facesOnly: the strip's voxels of planes -1 and BS, from the blocks below and above
+  if constexpr (facesOnly<T, FK>()) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass wrote them
 #pragma unroll
-      for (int zi = 0; zi < 2; zi++) {
-        const int s = nbs[zi * 18 + 4];
-        if (s >= 0)
-          zOut[zi] = __ldcg(reinterpret_cast<const V4 *>((const T *)a.payload + (int64_t)s * C::VPB +
-                                                            ((zi ? 0 : BS - 1) * BS + ty) * BS + tx));
-        else if (s == -1) zOut[zi] = ldsRow(offOf(t.er));
-      }
+    for (int zi = 0; zi < 2; zi++) {
+      const int s = nbs[zi * 18 + 4];
+      if (s >= 0)
+        zOut[zi] = __ldcg(reinterpret_cast<const V4 *>((const T *)a.payload + (int64_t)s * C::VPB +
+                                                          ((zi ? 0 : BS - 1) * BS + ty) * BS + tx));
+      else if (s == -1) zOut[zi] = ldsRow(offOf(t.er));
     }
-    auto fetchOut = [&](int p, Raw &r) {  // z-halo plane -1 or BS; the stencils read no edge of its rows y-1, y+1
-      if constexpr (facesOnly<T, FK>()) {  // and the 7-point form only the strip itself
-        const int zi = p < 0 ? 0 : 1, pc = zi ? BS - 1 : 0;
-        need(pc);
-        r.c = nbs[zi * 18 + 4] == -2 ? ldsRow(offOf(t.blk + (pc * BS + ty) * BS + tx)) : zOut[zi];
-        r.m = r.p = r.c;
-        r.em = r.ec = r.ep = 0;
-        return;
-      }
-      const int zi = p < 0 ? 0 : 1, dzb = zi ? 1 : -1, pc = zi ? BS - 1 : 0;
+  }
+  auto fetchOut = [&](int p, Raw &r) {  // z-halo plane -1 or BS; the stencils read no edge of its rows y-1, y+1
+    if constexpr (facesOnly<T, FK>()) {  // and the 7-point form only the strip itself
+      const int zi = p < 0 ? 0 : 1, pc = zi ? BS - 1 : 0;
       need(pc);
-      auto row = [&](int y) -> V4 {
-        const T *q;
-        if (y >= 0 && y < BS) {
-          const int s = nbs[(dzb + 1) * 9 + 4];
-          q = s >= 0 ? t.zpl[zi] + y * BS + tx : s == -1 ? t.er : t.blk + (pc * BS + y) * BS + tx;
-        } else {
-          const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1, s = nbs[(dzb + 1) * 9 + (dy + 1) * 3 + 1];
-          q = s >= 0 ? t.zh[zi][dy < 0 ? 2 : 3] + tx : s == -1 ? t.er : t.blk + (pc * BS + yc) * BS + tx;
-        }
-        return ldsRow(offOf(q));
-      };
-      r.m = row(ty - 1);
-      r.c = row(ty);
-      r.p = row(ty + 1);
-      const int side = atFirst ? 0 : 1, s = nbs[(dzb + 1) * 9 + 3 + (side ? 2 : 0)];
-      r.ec = ldsEdge(offOf(s >= 0 ? t.zh[zi][side] + ty : s == -1 ? t.er : t.blk + (pc * BS + ty) * BS + (side ? BS - 1 : 0)));
-      r.em = r.ep = 0;
-    };
-    auto unpackRow = [](const V4 &v, float o[4]) {
-      if constexpr (sizeof(T) == 4) {
-        o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+      r.c = nbs[zi * 18 + 4] == -2 ? ldsRow(offOf(t.blk + (pc * BS + ty) * BS + tx)) : zOut[zi];
+      r.m = r.p = r.c;
+      r.em = r.ec = r.ep = 0;
+      return;
+    }
+    const int zi = p < 0 ? 0 : 1, dzb = zi ? 1 : -1, pc = zi ? BS - 1 : 0;
+    need(pc);
+    auto row = [&](int y) -> V4 {
+      const T *q;
+      if (y >= 0 && y < BS) {
+        const int s = nbs[(dzb + 1) * 9 + 4];
+        q = s >= 0 ? t.zpl[zi] + y * BS + tx : s == -1 ? t.er : t.blk + (pc * BS + y) * BS + tx;
       } else {
-        const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-        const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-        o[0] = lo.x; o[1] = lo.y; o[2] = hi.x; o[3] = hi.y;
+        const int dy = y < 0 ? -1 : 1, yc = dy < 0 ? 0 : BS - 1, s = nbs[(dzb + 1) * 9 + (dy + 1) * 3 + 1];
+        q = s >= 0 ? t.zh[zi][dy < 0 ? 2 : 3] + tx : s == -1 ? t.er : t.blk + (pc * BS + yc) * BS + tx;
       }
+      return ldsRow(offOf(q));
     };
-    auto edgeVal = [](E v) {
-      if constexpr (sizeof(T) == 4) return v;
-      else return __half2float(__ushort_as_half(v));
-    };
-    auto plane = [&](const Raw &r, PW &W) {
-      StripRows s;
-      unpackRow(r.m, s.m);
-      unpackRow(r.c, s.c);
-      unpackRow(r.p, s.p);
-      s.ec = edgeVal(r.ec);
-      s.em = s.ep = 0.0f;
-      if constexpr (kCorners) { s.em = edgeVal(r.em); s.ep = edgeVal(r.ep); }
-      planeOf(s, atFirst, atLast, W);
-    };
-    auto fetch = [&](int p, Raw &r) {
-      if (p < 0 || p >= BS) fetchOut(p, r);
-      else fetchIn(p, r);
-    };
-    Raw r;
-    fetch(zFirst - 1, r);
-    plane(r, Wa);
-    fetchIn(zFirst, r);
-    plane(r, Wb);
-    fetch(zFirst + 1, r);
-    plane(r, Wc);
-    // the rows of plane z+2 are read while plane z is computed, and become the window that
-    // plane z-1 leaves
-    auto stepD = [&](int z, PW &A, PW &B, PW &Cw) {
-      const bool more = z + 1 < zFirst + PZ;
-      if (more) fetch(z + 2, r);
-      emit(z, A, B, Cw);
-      if (more) plane(r, A);
-    };
-    if constexpr (FKK == (K_MCF | FK_EXACT) || PZ % 3 != 2) {
-#pragma unroll 1
-      for (int z = zFirst; z < zFirst + PZ; z++) {
-        stepD(z, Wa, Wb, Wc);
-        const PW w = Wa;
-        Wa = Wb;
-        Wb = Wc;
-        Wc = w;
-      }
-    } else {  // PZ = 3 n + 2
-#pragma unroll 1
-      for (int z = zFirst; z + 3 <= zFirst + PZ; z += 3) {
-        stepD(z, Wa, Wb, Wc);
-        stepD(z + 1, Wb, Wc, Wa);
-        stepD(z + 2, Wc, Wa, Wb);
-      }
-      stepD(zFirst + PZ - 2, Wa, Wb, Wc);
-      stepD(zFirst + PZ - 1, Wb, Wc, Wa);
+    r.m = row(ty - 1);
+    r.c = row(ty);
+    r.p = row(ty + 1);
+    const int side = atFirst ? 0 : 1, s = nbs[(dzb + 1) * 9 + 3 + (side ? 2 : 0)];
+    r.ec = ldsEdge(offOf(s >= 0 ? t.zh[zi][side] + ty : s == -1 ? t.er : t.blk + (pc * BS + ty) * BS + (side ? BS - 1 : 0)));
+    r.em = r.ep = 0;
+  };
+  // u16 to float without the slow conversion pipe: u under the exponent of 2^23 is 2^23 + u
+  auto u16Val = [](uint32_t w, uint32_t sel) {
+    return __fmul_rn(__fsub_rn(__uint_as_float(__byte_perm(w, 0x4b000000u, sel)), 8388608.0f), kU16ToF);
+  };
+  auto unpackRow = [&](const V4 &v, float o[4]) {
+    if constexpr (sizeof(T) == 4) {
+      o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    } else if constexpr (std::is_same<T, uint16_t>::value) {
+      o[0] = u16Val(v.x, 0x7610); o[1] = u16Val(v.x, 0x7632);
+      o[2] = u16Val(v.y, 0x7610); o[3] = u16Val(v.y, 0x7632);
+    } else {
+      const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
+      const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+      o[0] = lo.x; o[1] = lo.y; o[2] = hi.x; o[3] = hi.y;
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // let the next pass in
-    if (timedOut) {
-      atomicOr(a.status, 1);
-      for (int k = 0; k < NCH; k++) waitChunk(&bar[k]);  // no copy may land after exit
-    }
-    return;
+  };
+  auto edgeVal = [&](E v) {
+    if constexpr (sizeof(T) == 4) return v;
+    else if constexpr (std::is_same<T, uint16_t>::value) return u16Val(v, 0x7610);
+    else return __half2float(__ushort_as_half(v));
+  };
+  auto plane = [&](const Raw &r, PW &W) {
+    StripRows s;
+    unpackRow(r.m, s.m);
+    unpackRow(r.c, s.c);
+    unpackRow(r.p, s.p);
+    s.ec = edgeVal(r.ec);
+    s.em = s.ep = 0.0f;
+    if constexpr (kCorners) { s.em = edgeVal(r.em); s.ep = edgeVal(r.ep); }
+    planeOf(s, atFirst, atLast, W);
+  };
+  auto fetch = [&](int p, Raw &r) {
+    if (p < 0 || p >= BS) fetchOut(p, r);
+    else fetchIn(p, r);
+  };
+  Raw r;
+  fetch(zFirst - 1, r);
+  plane(r, Wa);
+  fetchIn(zFirst, r);
+  plane(r, Wb);
+  fetch(zFirst + 1, r);
+  plane(r, Wc);
+  // the rows of plane z+2 are read while plane z is computed, and become the window that
+  // plane z-1 leaves
+  auto step = [&](int z, PW &A, PW &B, PW &Cw) {
+    const bool more = z + 1 < zFirst + PZ;
+    if (more) fetch(z + 2, r);
+    emit(z, A, B, Cw);
+    if (more) plane(r, A);
+  };
+  // the window roles rotate every plane: (a,b,c) -> (b,c,a)
+#pragma unroll 1
+  for (int z = zFirst; z + 3 <= zFirst + PZ; z += 3) {
+    step(z, Wa, Wb, Wc);
+    step(z + 1, Wb, Wc, Wa);
+    step(z + 2, Wc, Wa, Wb);
   }
-  // The loop in one copy: the exact form is bound by instruction fetch when its planes are
-  // unrolled (16^3 blocks, 1000 a pass: 32.6 us unrolled, generic scalar form; 21.8 us rolled
-  // and packed), and a z-group has few planes.
-  constexpr bool ROLL = ZG > 1 || FKK == (K_MCF | FK_EXACT);
-  if constexpr (!ROLL) {
-    // planes -1, 0, 1 into the windows (warp-local ring slots 0/1)
-    fillZ(-1, wring);
-    fillInterior(0, wring + PLX);
-    __syncwarp();
-    window(wring, Wa);
-    window(wring + PLX, Wb);
-    __syncwarp();
-    fillInterior(1, wring);
-    loadRaw(2);
-    __syncwarp();
-    window(wring, Wc);
-    __syncwarp();
-    // The window roles rotate every plane: (a,b,c) -> (b,c,a).  The main loop runs
-    // the planes z whose planes z+2 and z+3 are interior, three at a time; the
-    // last planes follow with their kinds known at compile time.
-    constexpr int MAIN = 3 * ((BS - 3) / 3);
-#pragma unroll 1
-    for (int z = 0; z < MAIN; z += 3) {
-      step(Interior{}, z, Wa, Wb, Wc);
-      step(Interior{}, z + 1, Wb, Wc, Wa);
-      step(Interior{}, z + 2, Wc, Wa, Wb);
-    }
-    static_assert(BS - MAIN >= 3 && BS - MAIN <= 5, "tail of 3..5 planes");
-    auto tail = [&](auto zc) {
-      constexpr int z = decltype(zc)::value;
-      if constexpr (z < BS) {
-        constexpr int K = z + 3 < BS ? 0 : z + 2 < BS ? 3 : (z + 2 == BS ? 1 : 2);
-        using KT = std::integral_constant<int, K>;
-        constexpr int r = (z - MAIN) % 3;
-        if constexpr (r == 0) step(KT{}, z, Wa, Wb, Wc);
-        else if constexpr (r == 1) step(KT{}, z, Wb, Wc, Wa);
-        else step(KT{}, z, Wc, Wa, Wb);
-      }
-    };
-    tail(std::integral_constant<int, MAIN>{});
-    tail(std::integral_constant<int, MAIN + 1>{});
-    tail(std::integral_constant<int, MAIN + 2>{});
-    tail(std::integral_constant<int, MAIN + 3>{});
-    tail(std::integral_constant<int, MAIN + 4>{});
-  } else {
-    // plane p = -1 .. BS into a ring slot
-    auto stagePlane = [&](int p, float *slot) {
-      if (p < 0 || p >= BS) fillZ(p, slot);
-      else fillInterior(p, slot);
-    };
-    stagePlane(zFirst - 1, wring);
-    fillInterior(zFirst, wring + PLX);
-    __syncwarp();
-    window(wring, Wa);
-    window(wring + PLX, Wb);
-    __syncwarp();
-    stagePlane(zFirst + 1, wring);
-    __syncwarp();
-    window(wring, Wc);
-    __syncwarp();
-#pragma unroll 1
-    for (int i = 0; i < PZ; i++) {
-      float *slot = wring + ((i + 1) & 1) * PLX;
-      const bool more = i + 1 < PZ;
-      if (more) stagePlane(zFirst + i + 2, slot);
-      __syncwarp();
-      emit(zFirst + i, Wa, Wb, Wc);
-      Wa = Wb;
-      Wb = Wc;
-      if (more) window(slot, Wc);
-    }
-  }
+  constexpr int PT = PZ - PZ % 3;
+  if constexpr (PZ % 3 > 0) step(zFirst + PT, Wa, Wb, Wc);
+  if constexpr (PZ % 3 > 1) step(zFirst + PT + 1, Wb, Wc, Wa);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // let the next pass in
   if (timedOut) {
     atomicOr(a.status, 1);
@@ -837,7 +584,7 @@ static int zGroups(int n, int ki) {
   constexpr int kSm = 152;
   if constexpr (BS == 16) {
     if (n <= 2 * kSm) return 4;
-    return ki == kKernMcfExact && n <= 4 * kSm ? 2 : 1;
+    return (ki == kKernMcfExact || ki == kKernMcf || ki == kKernMcfClamp) && n <= 4 * kSm ? 2 : 1;
   } else {
     return ki == kKernMcfExact && (sizeof(T) == 4 || n <= kSm) ? 2 : 1;
   }
@@ -846,7 +593,7 @@ static int zGroups(int n, int ki) {
 template <typename T, int BS, int FK, int ZG>
 static cudaError_t launchPassT(const ColorArgs &a, unsigned blocks, cudaStream_t st) {
   const auto kern = kSweepColor<T, BS, FK, ZG>;
-  constexpr size_t smem = colorSmemBytes<T, BS, FK, ZG>();
+  constexpr size_t smem = colorSmemBytes<T, BS, FK>();
   static bool attrSet = false;
   if (!attrSet) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -870,8 +617,11 @@ template <typename T, int BS>
 static cudaError_t launchPass(const ColorArgs &a, int ki, int zg, unsigned blocks, cudaStream_t st) {
   constexpr int ZS = BS == 16 ? 4 : 1;  // the small passes' groups (generic and fast forms)
   switch (ki) {
-    case kKernMcf: return zg > 1 ? launchPassT<T, BS, K_MCF, ZS>(a, blocks, st) : launchPassT<T, BS, K_MCF, 1>(a, blocks, st);
+    case kKernMcf:
+      if constexpr (ZS > 1) if (zg == 2) return launchPassT<T, BS, K_MCF, 2>(a, blocks, st);
+      return zg > 1 ? launchPassT<T, BS, K_MCF, ZS>(a, blocks, st) : launchPassT<T, BS, K_MCF, 1>(a, blocks, st);
     case kKernMcfClamp:
+      if constexpr (ZS > 1) if (zg == 2) return launchPassT<T, BS, K_MCF | FK_CLAMP, 2>(a, blocks, st);
       return zg > 1 ? launchPassT<T, BS, K_MCF | FK_CLAMP, ZS>(a, blocks, st)
                     : launchPassT<T, BS, K_MCF | FK_CLAMP, 1>(a, blocks, st);
     case kKernJacobi:

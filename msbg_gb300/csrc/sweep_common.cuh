@@ -153,55 +153,7 @@ struct PlaneMcfX {
   float r0[4], r1[6], r2[4], h0, h5;
 };
 
-// Reads one plane from the FP32 ring: row0 = row y-1 at column x-1; rows RS apart.
-template <int RS>
-__device__ __forceinline__ void loadPlane(const float *row0, PlaneRaw &P) {
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    const float *row = row0 + r * RS;
-    const float4 m = *reinterpret_cast<const float4 *>(row + 1);
-    P.w[r][0] = row[0]; P.w[r][1] = m.x; P.w[r][2] = m.y; P.w[r][3] = m.z; P.w[r][4] = m.w; P.w[r][5] = row[5];
-  }
-}
-template <int RS>
-__device__ __forceinline__ void loadRow1(const float *row0, float (&r1)[6]) {
-  const float *row = row0 + RS;
-  const float4 m = *reinterpret_cast<const float4 *>(row + 1);
-  r1[0] = row[0]; r1[1] = m.x; r1[2] = m.y; r1[3] = m.z; r1[4] = m.w; r1[5] = row[5];
-}
-template <int RS>
-__device__ __forceinline__ void loadPlane(const float *row0, PlaneMcf &P) {
-  loadRow1<RS>(row0, P.r1);
-  const float4 u = *reinterpret_cast<const float4 *>(row0 + 1);
-  const float4 v = *reinterpret_cast<const float4 *>(row0 + 2 * RS + 1);
-  const float2 d01 = sub2(pr(v.x, v.y), pr(u.x, u.y)), d23 = sub2(pr(v.z, v.w), pr(u.z, u.w));
-  const float2 s01 = add2(pr(u.x, u.y), pr(v.x, v.y)), s23 = add2(pr(u.z, u.w), pr(v.z, v.w));
-  P.dy[0] = row0[2 * RS] - row0[0];
-  P.dy[1] = d01.x; P.dy[2] = d01.y; P.dy[3] = d23.x; P.dy[4] = d23.y;
-  P.dy[5] = row0[2 * RS + 5] - row0[5];
-  P.sy[0] = s01.x; P.sy[1] = s01.y; P.sy[2] = s23.x; P.sy[3] = s23.y;
-}
-template <int RS>
-__device__ __forceinline__ void loadPlane(const float *row0, PlaneJac &P) {
-  loadRow1<RS>(row0, P.r1);
-  const float4 u = *reinterpret_cast<const float4 *>(row0 + 1);
-  const float4 v = *reinterpret_cast<const float4 *>(row0 + 2 * RS + 1);
-  const float2 s01 = add2(pr(u.x, u.y), pr(v.x, v.y)), s23 = add2(pr(u.z, u.w), pr(v.z, v.w));
-  P.sy[0] = s01.x; P.sy[1] = s01.y; P.sy[2] = s23.x; P.sy[3] = s23.y;
-}
-
-template <int RS>
-__device__ __forceinline__ void loadPlane(const float *row0, PlaneMcfX &P) {
-  loadRow1<RS>(row0, P.r1);
-  const float4 u = *reinterpret_cast<const float4 *>(row0 + 1);
-  const float4 v = *reinterpret_cast<const float4 *>(row0 + 2 * RS + 1);
-  P.r0[0] = u.x; P.r0[1] = u.y; P.r0[2] = u.z; P.r0[3] = u.w;
-  P.r2[0] = v.x; P.r2[1] = v.y; P.r2[2] = v.z; P.r2[3] = v.w;
-  P.h0 = __fmul_rn(0.5f, __fsub_rn(row0[2 * RS], row0[0]));
-  P.h5 = __fmul_rn(0.5f, __fsub_rn(row0[2 * RS + 5], row0[5]));
-}
-
-// The same planes from a thread's own three rows (four values each: y-1, y, y+1) and, in the
+// The planes from a thread's own three rows (four values each: y-1, y, y+1) and, in the
 // lanes that hold a block row's first and last strip (edge), one value beyond it per row;
 // the other lanes' values beyond the strip are their neighbours' (a row's strips lie in
 // consecutive lanes).
@@ -213,6 +165,13 @@ __device__ __forceinline__ void sides(float first, float last, float beyond, boo
   const float l = __shfl_up_sync(0xffffffffu, last, 1), r = __shfl_down_sync(0xffffffffu, first, 1);
   left = atFirst ? beyond : l;
   right = atLast ? beyond : r;
+}
+__device__ __forceinline__ void planeOf(const StripRows &s, bool atFirst, bool atLast, PlaneRaw &P) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) { P.w[0][i + 1] = s.m[i]; P.w[1][i + 1] = s.c[i]; P.w[2][i + 1] = s.p[i]; }
+  sides(s.m[0], s.m[3], s.em, atFirst, atLast, P.w[0][0], P.w[0][5]);
+  sides(s.c[0], s.c[3], s.ec, atFirst, atLast, P.w[1][0], P.w[1][5]);
+  sides(s.p[0], s.p[3], s.ep, atFirst, atLast, P.w[2][0], P.w[2][5]);
 }
 __device__ __forceinline__ void planeOf(const StripRows &s, bool atFirst, bool atLast, PlaneJac &P) {
   P.r1[1] = s.c[0]; P.r1[2] = s.c[1]; P.r1[3] = s.c[2]; P.r1[4] = s.c[3];
