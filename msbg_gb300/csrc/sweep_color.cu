@@ -254,6 +254,7 @@ constexpr size_t colorSmemBytes() {
 template <typename T, int BS, int FK, int ZG>
 constexpr int sweepCtas() {  // resident CTAs to leave registers for
   constexpr int nt = ColorSweep<T, BS>::NT * ZG;
+  if ((FK & ~FK_CLAMP) == K_JACOBI && BS == 16 && ZG == 4) return 4;
   return facesOnly<T, FK>() && BS == 32 ? 3 : nt <= 256 ? 512 / nt : 1;
 }
 
@@ -571,20 +572,22 @@ enum { kKernGeneric, kKernMcf, kKernMcfClamp, kKernJacobi, kKernJacobiClamp, kKe
 
 // z-groups per CTA of a pass of n blocks.  A pass is as long as one block takes while its
 // CTAs fit the chip at once (152 SMs), and more groups shorten a block; they cost every
-// group two more planes to stage, so a pass of several waves takes fewer.  Measured, us a
-// pass for 1 / 2 / 4 groups (FP32, 16^3 blocks): exact MCF 11.0 / 7.9 / 6.6 at 64 blocks,
-// 12.2 / 9.7 / 8.3 at 216, 15.4 / 12.8 / 16.3 at 512, 21.8 / 23.3 / 30.6 at 1000; fast MCF
-// 6.9 / 6.8 / 6.1 at 64, 11.6 / 11.0 / 14.9 at 512; fast Jacobi 5.7 / 5.7 / 5.3 at 64.
-// Two 4-group CTAs or four 2-group CTAs (registers) share an SM.  On 32^3 blocks the exact
-// form takes two groups up to one block per SM (24.2 -> 19.2 us, FP16, 64 blocks) and,
-// with FP32 storage, whose 145 KB of staging leave one CTA per SM, always (96.8 -> 80.9 us
-// at 512 blocks); the fast forms are not faster with two.
+// group two more planes to read, so a pass of several waves takes fewer.  Two 4-group or four
+// 2-group CTAs (registers) share an SM, four 4-group ones of the fast Jacobi.  Measured, us a
+// pass for 1 / 2 / 4 groups (FP32, 16^3 blocks): exact MCF 9.4 / 7.3 / 5.2 at 64 blocks, 10.2 /
+// 7.9 / 6.2 at 216, 12.5 / 10.6 / 12.6 at 512, 14.9 / 17.1 / 18.5 at 729; fast MCF 6.8 / 5.7 /
+// 4.6 at 64, 9.3 / 8.6 / 11.0 at 512, 11.2 / 14.4 / 16.9 at 729; fast Jacobi for 1 / 4: 5.3 /
+// 4.1 at 64, 6.7 / 5.6 at 512, 8.2 / 10.5 at 729.  On 32^3 blocks the exact form takes two
+// groups up to one block per SM (FP16, 64 blocks: 18.4 -> 15.7; 216 blocks: 26.7 against 32.0)
+// and, with FP32 storage, whose 145 KB of staging leave one CTA per SM, always (76.3 -> 67.9 at
+// 512 blocks).
 template <typename T, int BS>
 static int zGroups(int n, int ki) {
   constexpr int kSm = 152;
   if constexpr (BS == 16) {
     if (n <= 2 * kSm) return 4;
-    return (ki == kKernMcfExact || ki == kKernMcf || ki == kKernMcfClamp) && n <= 4 * kSm ? 2 : 1;
+    if (n > 4 * kSm || ki == kKernGeneric) return 1;
+    return ki == kKernJacobi || ki == kKernJacobiClamp ? 4 : 2;
   } else {
     return ki == kKernMcfExact && (sizeof(T) == 4 || n <= kSm) ? 2 : 1;
   }
