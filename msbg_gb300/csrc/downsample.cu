@@ -22,27 +22,30 @@
 // new planes per coarse plane, so each fine plane is read from memory once; the
 // loads of the next two planes are in flight while the current two are used.  Each
 // thread carries its 16 partial sums of the coarse plane above in registers.
-// Bytes: S per fine cell read (plus the halo), 4 per coarse cell written, i.e.
-// HBM-bound at S + 1/2 bytes per fine cell.
+// The planes in flight are kept as stored and widened when they are put into the ring:
+// a conversion at the load would wait for it.  The thread's ring cells are looked up
+// once for the block's own z-layer, the sums run in column pairs on the packed FP32
+// pipe (the same operations per column).  Floor: S bytes per fine cell read, 4 per
+// coarse cell written (236 M FP16 cells: 85 us); measured 322 us with per-plane lookups
+// and conversions at the load, 274 with the lookups and the pairs alone, 199 with all.
+// Bound now: the latency of a CTA's steps (64 registers, half the warps an SM holds).
 #include "internal.cuh"
 
 namespace msbg {
 
-// Four consecutive values of a block row as floats (one 8- or 16-byte load; x is a
-// multiple of 4), converted as Store<T>::load does.
-template <typename T> __device__ __forceinline__ void ldQuad(const T *p, float v[4]);
-template <> __device__ __forceinline__ void ldQuad<float>(const float *p, float v[4]) {
-  const float4 q = *reinterpret_cast<const float4 *>(p);
+// Four consecutive values of a block row as stored (one 8- or 16-byte load; x is a multiple of
+// 4), and as floats, converted as Store<T>::load does.
+template <typename T> struct Quad { using V = uint2; };
+template <> struct Quad<float> { using V = float4; };
+__device__ __forceinline__ void quadVals(const float4 &q, float v[4], const float *) {
   v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
-template <> __device__ __forceinline__ void ldQuad<__half>(const __half *p, float v[4]) {
-  const uint2 q = *reinterpret_cast<const uint2 *>(p);
+__device__ __forceinline__ void quadVals(const uint2 &q, float v[4], const __half *) {
   const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&q.x));
   const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&q.y));
   v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
 }
-template <> __device__ __forceinline__ void ldQuad<uint16_t>(const uint16_t *p, float v[4]) {
-  const uint2 q = *reinterpret_cast<const uint2 *>(p);
+__device__ __forceinline__ void quadVals(const uint2 &q, float v[4], const uint16_t *) {
   v[0] = __fmul_rn((float)(q.x & 0xffffu), kU16ToF);
   v[1] = __fmul_rn((float)(q.x >> 16), kU16ToF);
   v[2] = __fmul_rn((float)(q.y & 0xffffu), kU16ToF);
@@ -82,30 +85,62 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   // the ring slot.
   constexpr int NI = BS * BS / 4, NR = 4 * (BS + 1), PR = (NR + NT - 1) / NT;
   static_assert(NI <= NT, "one interior quad per thread");
+  // a plane's values as stored: a conversion here would wait for the loads it follows
   struct Plane {
-    float in[4], ring[PR];
+    typename Quad<T>::V in;
+    T ring[PR];
   };
+  const T zero = T(0.0f);  // the empty value
+  // ring cell e: rows 0 and H-1 (e < 2H), then columns 0 and H-1 of rows 1..H-2
+  auto ringAt = [](int e, int &r, int &c) {
+    if (e < 2 * H) { r = e < H ? 0 : H - 1; c = e < H ? e : e - H; }
+    else { const int f = e - 2 * H; r = 1 + (f >> 1); c = (f & 1) ? H - 1 : 0; }
+  };
+  // the thread's ring cells in the block's own z-layer: their source in plane 0 (null: an empty
+  // block) and their place in a ring slot (-1: none)
+  const T *ringSrc[PR];
+  int ringDst[PR];
+#pragma unroll
+  for (int k = 0; k < PR; k++) {
+    const int e = tid + k * NT;
+    ringSrc[k] = nullptr;
+    ringDst[k] = -1;
+    if (e < NR) {
+      int r, c;
+      ringAt(e, r, c);
+      ringDst[k] = r * H + c;
+      const int gy = min(max((by << L) + r - 1, 0), sy - 1), gx = min(max((bx << L) + c - 1, 0), sx - 1);
+      const int sn = nbs[9 + 1 + ((gy >> L) - by + 1) * 3 + (gx >> L) - bx];
+      if (sn >= 0) ringSrc[k] = pay + ((int64_t)sn << (3 * L)) + ((gy & m) << L) + (gx & m);
+    }
+  }
+  const T *quadSrc = pay + ((int64_t)t << (3 * L)) + 4 * tid;
   auto fetch = [&](int p, Plane &v) {
+    if (p >= 0 && p < BS) {
+      if (tid < NI) v.in = *reinterpret_cast<const typename Quad<T>::V *>(quadSrc + (p << (2 * L)));
+#pragma unroll
+      for (int k = 0; k < PR; k++)
+        v.ring[k] = ringSrc[k] ? ringSrc[k][p << (2 * L)] : zero;
+      return;
+    }
     const int gz = min(max((bz << L) + p, 0), sz - 1);
     const int nz = ((gz >> L) - bz + 1) * 9 + 1;
     const int64_t zoff = (int64_t)(gz & m) << (2 * L);
     if (tid < NI) {
       const int sc = nbs[nz + 3];  // the block above / below (or the own block)
-      v.in[0] = v.in[1] = v.in[2] = v.in[3] = 0.0f;
-      if (sc >= 0) ldQuad<T>(pay + ((int64_t)sc << (3 * L)) + zoff + 4 * tid, v.in);
+      v.in = {};
+      if (sc >= 0) v.in = *reinterpret_cast<const typename Quad<T>::V *>(pay + ((int64_t)sc << (3 * L)) + zoff + 4 * tid);
     }
 #pragma unroll
     for (int k = 0; k < PR; k++) {
       const int e = tid + k * NT;
-      v.ring[k] = 0.0f;  // the empty value
+      v.ring[k] = zero;
       if (e < NR) {
-        // ring cell e: rows 0 and H-1 (e < 2H), then columns 0 and H-1 of rows 1..H-2
         int r, c;
-        if (e < 2 * H) { r = e < H ? 0 : H - 1; c = e < H ? e : e - H; }
-        else { const int f = e - 2 * H; r = 1 + (f >> 1); c = (f & 1) ? H - 1 : 0; }
+        ringAt(e, r, c);
         const int gy = min(max((by << L) + r - 1, 0), sy - 1), gx = min(max((bx << L) + c - 1, 0), sx - 1);
         const int sn = nbs[nz + ((gy >> L) - by + 1) * 3 + (gx >> L) - bx];
-        if (sn >= 0) v.ring[k] = Store<T>::load(pay + ((int64_t)sn << (3 * L)) + zoff + ((gy & m) << L) + (gx & m));
+        if (sn >= 0) v.ring[k] = pay[((int64_t)sn << (3 * L)) + zoff + ((gy & m) << L) + (gx & m)];
       }
     }
   };
@@ -114,39 +149,35 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
     if (tid < NI) {
       const int r = (4 * tid) >> L, c = (4 * tid) & m;
       float *q = dst + (r + 1) * H + c + 1;
+      float in[4];
+      quadVals(v.in, in, (const T *)nullptr);
 #pragma unroll
-      for (int k = 0; k < 4; k++) q[k] = v.in[k];
+      for (int k = 0; k < 4; k++) q[k] = in[k];
     }
 #pragma unroll
-    for (int k = 0; k < PR; k++) {
-      const int e = tid + k * NT;
-      if (e < NR) {
-        int r, c;
-        if (e < 2 * H) { r = e < H ? 0 : H - 1; c = e < H ? e : e - H; }
-        else { const int f = e - 2 * H; r = 1 + (f >> 1); c = (f & 1) ? H - 1 : 0; }
-        dst[r * H + c] = v.ring[k];
-      }
-    }
+    for (int k = 0; k < PR; k++)
+      if (ringDst[k] >= 0) dst[ringDst[k]] = Store<T>::load(&v.ring[k]);
   };
   const bool own = tid < CB * CB;
   const int vx = tid & (CB - 1), vy = tid / CB;
-  // exact weights k1[k] k1[j] k1[i] / 512 of (plane k, row j, column i)
-  auto wgt = [](int k, int j, int i) {
+  // exact weights k1[k] k1[j] k1[i] / 512 of (plane k, row j, columns i = 2h, 2h + 1)
+  auto wgt = [](int k, int j, int h) {
     const float k1[4] = {1.f, 3.f, 3.f, 1.f};
-    return k1[k] * k1[j] * k1[i] / 512.0f;
+    return make_float2(k1[k] * k1[j] * k1[2 * h] / 512.0f, k1[k] * k1[j] * k1[2 * h + 1] / 512.0f);
   };
   // row j (fine row 2vy-1+j, columns 2vx-1 .. 2vx+2) of fine plane p
-  auto row = [&](int p, int j, float (&r)[4]) {
+  auto row = [&](int p, int j, float2 (&r)[2]) {
     const float *src = st + ((p + 1) & 3) * HH + (2 * vy + j) * H + 2 * vx;
-    const float2 a = *reinterpret_cast<const float2 *>(src);
-    const float2 b = *reinterpret_cast<const float2 *>(src + 2);
-    r[0] = a.x; r[1] = a.y; r[2] = b.x; r[3] = b.y;
+    r[0] = *reinterpret_cast<const float2 *>(src);
+    r[1] = *reinterpret_cast<const float2 *>(src + 2);
   };
   // Coarse plane vz reads fine planes 2vz-1 .. 2vz+2 (k = 0..3).  The accumulators of
   // plane vz over k = 0, 1 come from the previous pair of fine planes; the pair
   // (2vz+1, 2vz+2) completes them (k = 2, 3) and starts those of plane vz+1.  The
   // next pair's loads are in flight while a pair is used.
-  float acc[4][4], part = 0.0f;  // acc[j][i] over k = 0, 1; part: the children sum in plane 2vz
+  const float2 zero2 = make_float2(0.0f, 0.0f);
+  float2 acc[4][2];  // acc[j][h]: columns 2h, 2h + 1 over k = 0, 1
+  float part = 0.0f;  // part: the children sum in plane 2vz
   // Fine-plane pairs go through two register sets (A: pairs of even coarse planes, B:
   // odd), so the loads of the next two pairs are in flight while a pair is used.
   Plane va, vb, vc, vd;
@@ -162,14 +193,14 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   if (own) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      float r0[4], r1[4];
+      float2 r0[2], r1[2];
       row(-1, j, r0);
       row(0, j, r1);
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        if (!SIMPLE) acc[j][i] = __fmaf_rn(wgt(1, j, i), r1[i], __fmaf_rn(wgt(0, j, i), r0[i], 0.0f));
-      if (SIMPLE && j == 1) part = __fadd_rn(r1[1], r1[2]);
-      if (SIMPLE && j == 2) part = __fadd_rn(__fadd_rn(part, r1[1]), r1[2]);
+      for (int h = 0; h < 2; h++)
+        if (!SIMPLE) acc[j][h] = __ffma2_rn(wgt(1, j, h), r1[h], __ffma2_rn(wgt(0, j, h), r0[h], zero2));
+      if (SIMPLE && j == 1) part = __fadd_rn(r1[0].y, r1[1].x);
+      if (SIMPLE && j == 2) part = __fadd_rn(__fadd_rn(part, r1[0].y), r1[1].x);
     }
   }
   // one coarse plane from the pair (p, q) of fine planes 2vz+1, 2vz+2
@@ -184,27 +215,28 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
       fetch(2 * vz + 6, q);
     }
     if (!own) return;
-    float T4[4], sum = part, npart = 0.0f;
+    float2 T2[2];
+    float sum = part, npart = 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      float r2[4], r3[4];
+      float2 r2[2], r3[2];
       row(2 * vz + 1, j, r2);
       row(2 * vz + 2, j, r3);
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
+      for (int h = 0; h < 2; h++) {
         if (SIMPLE) break;
-        const float S = __fmaf_rn(wgt(3, j, i), r3[i], __fmaf_rn(wgt(2, j, i), r2[i], acc[j][i]));
-        T4[i] = j == 0 ? S : __fadd_rn(T4[i], S);
-        acc[j][i] = __fmaf_rn(wgt(1, j, i), r3[i], __fmaf_rn(wgt(0, j, i), r2[i], 0.0f));
+        const float2 S = __ffma2_rn(wgt(3, j, h), r3[h], __ffma2_rn(wgt(2, j, h), r2[h], acc[j][h]));
+        T2[h] = j == 0 ? S : __fadd2_rn(T2[h], S);
+        acc[j][h] = __ffma2_rn(wgt(1, j, h), r3[h], __ffma2_rn(wgt(0, j, h), r2[h], zero2));
       }
       if (SIMPLE && (j == 1 || j == 2)) {  // children in plane 2vz+1 (this cell) and 2vz+2 (the next)
-        sum = __fadd_rn(__fadd_rn(sum, r2[1]), r2[2]);
-        npart = j == 1 ? __fadd_rn(r3[1], r3[2]) : __fadd_rn(__fadd_rn(npart, r3[1]), r3[2]);
+        sum = __fadd_rn(__fadd_rn(sum, r2[0].y), r2[1].x);
+        npart = j == 1 ? __fadd_rn(r3[0].y, r3[1].x) : __fadd_rn(__fadd_rn(npart, r3[0].y), r3[1].x);
       }
     }
     part = npart;
     const float val = SIMPLE ? __fmul_rn(sum, 0.125f)
-                             : __fadd_rn(__fadd_rn(T4[0], T4[1]), __fadd_rn(T4[2], T4[3]));
+                             : __fadd_rn(__fadd_rn(T2[0].x, T2[0].y), __fadd_rn(T2[1].x, T2[1].y));
     out[(int64_t)t * CB * CB * CB + ((int64_t)vz * CB + vy) * CB + vx] = val;
   };
   static_assert(CB % 2 == 0, "coarse planes in pairs");
