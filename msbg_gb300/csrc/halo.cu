@@ -263,7 +263,9 @@ __global__ void __launch_bounds__(kHaloThreads, 8) kFillHalo(HaloArgs a) {
 // per plane; looking every row up (the table, but no constant step) was bound by issue as
 // well, 87 k warp instructions a block against 37 k.  Measured (FP16, bs 32, halo 1, a
 // coarser level beside, 2,565 blocks, 540 MB): 233 us plane-wise, 236 with every row looked
-// up, 190 so; bound now by the loads' latency (45% of issue slots, 30 warps per SM).
+// up, 190 so, and 147 once no load is touched before its pair is written (the halo column's
+// 16-bit value was merged into a cleared word right away, and the warp waited for it).  Bound
+// now by the loads' latency.
 template <typename T>
 struct HaloEntry {
   const T *p;           // null: the constant c
@@ -410,9 +412,8 @@ __global__ void __launch_bounds__(kHaloRowThreads, 4) kFillHaloRows(HaloArgs a) 
       if (hasS) {
         at(ss, xs, ys, 2 * k + zs);
         if (ss.kind) {
-          const T v = *ss.p;
-          t.s = 0;
-          memcpy(&t.s, &v, sizeof(T));
+          if constexpr (sizeof(T) == 4) t.s = __ldg(reinterpret_cast<const uint32_t *>(ss.p));
+          else t.s = __ldg(reinterpret_cast<const unsigned short *>(ss.p));
         } else {
           memcpy(&t.s, &ss.c, 4);
         }
