@@ -114,19 +114,15 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
     const int64_t base = (int64_t)s << (3 * L);
     const int64_t c = base + ((int64_t)((lz << L) + ly) << L) + lx;
 
-    RawRow<V, CPT> xv, dv, cxv, cyv, czv, ym, yq, zm, zq, cyu, czu;
+    // All loads as stored, the conversions after the last one (a conversion waits for its
+    // load); the x neighbours, which may need a block's table entry first, come last.
+    RawRow<V, CPT> xv, dv, cxv, cyv, czv, ym, yq, zm, zq, cyu, czu, bRow;
     xv.ld(x + c);
     dv.ld(d + c);
     cxv.ld(cx + c);
     cyv.ld(cy + c);
     czv.ld(cz + c);
-    float xl = 0.f, xr = 0.f, cxr = 0.f;
-    {
-      const int64_t j = lx > 0 ? c - 1 : cellAt(g, s, lx - 1, ly, lz);
-      if (j >= 0) xl = ldv(x + j);
-      const int64_t k = lx + CPT < bs ? c + CPT : cellAt(g, s, lx + CPT, ly, lz);
-      if (k >= 0) { xr = ldv(x + k); cxr = ldv(cx + k); }
-    }
+    if constexpr (MODE > 0) bRow.ld(b + c);
     {
       const int64_t j = ly > 0 ? c - sy : cellAt(g, s, lx, ly - 1, lz);
       if (j >= 0) ym.ld(x + j); else ym.zero();
@@ -141,14 +137,20 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
       if (k >= 0) { zq.ld(x + k); czu.ld(cz + k); }
       else { zq.zero(); czu.zero(); }
     }
+    V xlV = V(0.f), xrV = V(0.f), cxrV = V(0.f);
+    {
+      const int64_t j = lx > 0 ? c - 1 : cellAt(g, s, lx - 1, ly, lz);
+      const int64_t k = lx + CPT < bs ? c + CPT : cellAt(g, s, lx + CPT, ly, lz);
+      if (j >= 0) xlV = x[j];
+      if (k >= 0) { xrV = x[k]; cxrV = cx[k]; }
+    }
+    const float xl = ldv(&xlV), xr = ldv(&xrV), cxr = ldv(&cxrV);
     float r[CPT];
     if constexpr (MODE == 2) {
       static_assert(MODE != 2 || CPT == 4, "the checked residual runs on FP32 storage");
       // r = b - A x in double-float arithmetic: every product split exactly into
       // a rounded part and its error (fma), the running sum kept exact with
       // TwoSum and the errors gathered in a second float; then sum r^2, b^2.
-      float bv[CPT];
-      ldRow<CPT>(b + c, bv);
       float rq = 0.f, bq = 0.f;
 #pragma unroll
       for (int i = 0; i < CPT; i++) {
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
         const float cxp = i == CPT - 1 ? cxr : cxv[i + 1];
         const float fa[7] = {-dv[i], cxv[i], cxp, cyv[i], cyu[i], czv[i], czu[i]};
         const float fb[7] = {xv[i], xm1, xp1, ym[i], yq[i], zm[i], zq[i]};
-        float S = bv[i], E = 0.f;
+        float S = bRow[i], E = 0.f;
 #pragma unroll
         for (int t = 0; t < 7; t++) {
           const float h = __fmul_rn(fa[t], fb[t]);
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
         }
         r[i] = __fadd_rn(S, E);
         rq = fmaf(r[i], r[i], rq);
-        bq = fmaf(bv[i], bv[i], bq);
+        bq = fmaf(bRow[i], bRow[i], bq);
       }
       if (act) {
         dot += (double)rq;
@@ -197,11 +199,9 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
       a -= czu[i] * zq[i];
       r[i] = a;
     }
-    if (MODE == 1) {
-      float bv[CPT];
-      ldRow<CPT>(b + c, bv);
+    if constexpr (MODE == 1) {
 #pragma unroll
-      for (int i = 0; i < CPT; i++) r[i] = bv[i] - r[i];
+      for (int i = 0; i < CPT; i++) r[i] = bRow[i] - r[i];
     }
     if (dotPartial && act) {
       float qd = 0.f;  // four products in FP32, then FP64 accumulation
