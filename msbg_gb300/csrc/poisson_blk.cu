@@ -494,40 +494,51 @@ __global__ void __launch_bounds__(tileThreads<BS>(), 2)
   }
   // while the boxes fly: the x halo columns (x = -1, x = TX) and cx at x = TX by
   // plain loads (face cell (y, z) = (q % TY, q / TY)), coarse corrections
+  // Values stay as stored until the boxes have landed: a conversion waits for its load, and
+  // the loads behind it for the conversion.
   constexpr int NXF = (S::CX2 + TXY - 1) / TXY;
-  float xlo[NXF], xhi[NXF];
+  const V zeroV = V(0.f);
+  V xloV[NXF], xhiV[NXF], xloC[NXF], xhiC[NXF];  // values and coarse corrections
   using CxT = std::conditional_t<S::H, V, float>;
   CxT *cxhi = reinterpret_cast<CxT *>(tb + S::CXHI);
+  V chi[NXF];
 #pragma unroll
   for (int i = 0; i < NXF; i++) {
     const int q = r + i * TXY;
-    xlo[i] = xhi[i] = 0.f;
+    xloV[i] = xhiV[i] = xloC[i] = xhiC[i] = chi[i] = zeroV;
     if (valid && q < S::CX2) {
       const int j = q % TY, kk = q / TY;
       const int64_t lo = cellAt(g, s, ox - 1, oy + j, oz + kk);
       const int64_t hi = cellAt(g, s, ox + TX, oy + j, oz + kk);
-      CxT chi = CxT(0.f);
-      if (lo >= 0 && !haloZero) xlo[i] = ldv(x + lo) + (haloCorr ? ldv(xc + parentOf(lo, L)) : 0.f);
-      if (hi >= 0) {
-        if constexpr (S::H) chi = cxg[hi]; else chi = ldv(cxg + hi);
-        if (!haloZero) xhi[i] = ldv(x + hi) + (haloCorr ? ldv(xc + parentOf(hi, L)) : 0.f);
+      if (hi >= 0) chi[i] = cxg[hi];
+      if (!haloZero) {
+        if (lo >= 0) xloV[i] = x[lo];
+        if (hi >= 0) xhiV[i] = x[hi];
+        if (haloCorr) {
+          if (lo >= 0) xloC[i] = xc[parentOf(lo, L)];
+          if (hi >= 0) xhiC[i] = xc[parentOf(hi, L)];
+        }
       }
-      cxhi[q] = chi;
     }
   }
-  float corr[TZ / 2], czc0 = 0.f, czc1 = 0.f;
+  V corrV[TZ / 2], czc0V = zeroV, czc1V = zeroV;
 #pragma unroll
-  for (int z = 0; z < TZ / 2; z++) corr[z] = 0.f;
+  for (int z = 0; z < TZ / 2; z++) corrV[z] = zeroV;
   if (valid && ownCorr) {
     const int Lc = L - 1;
     const int64_t pb = ((int64_t)s << (3 * Lc)) + ((ox + tx) >> 1) + ((int64_t)((oy + ty) >> 1) << Lc);
 #pragma unroll
-    for (int z = 0; z < TZ / 2; z++) corr[z] = ldv(xc + pb + ((int64_t)((oz >> 1) + z) << (2 * Lc)));
+    for (int z = 0; z < TZ / 2; z++) corrV[z] = xc[pb + ((int64_t)((oz >> 1) + z) << (2 * Lc))];
   }
   if (valid && haloCorr) {  // the z-halo cells of this column
     const int64_t j2 = cellAt(g, s, ox + tx, oy + ty, oz - 1), j3 = cellAt(g, s, ox + tx, oy + ty, oz + TZ);
-    if (j2 >= 0) czc0 = ldv(xc + parentOf(j2, L));
-    if (j3 >= 0) czc1 = ldv(xc + parentOf(j3, L));
+    if (j2 >= 0) czc0V = xc[parentOf(j2, L)];
+    if (j3 >= 0) czc1V = xc[parentOf(j3, L)];
+  }
+#pragma unroll
+  for (int i = 0; i < NXF; i++) {
+    const int q = r + i * TXY;
+    if (q < S::CX2) cxhi[q] = (CxT)chi[i];
   }
   // wait for the boxes (bounded): one warp polls the barrier, the others sleep in
   // __syncthreads, which also publishes the landed data to them; the decision is
@@ -545,6 +556,15 @@ __global__ void __launch_bounds__(tileThreads<BS>(), 2)
       if (mbarTryWait(bar, 0)) break;  // no copy may land after exit
     return;
   }
+  float xlo[NXF], xhi[NXF], corr[TZ / 2];
+#pragma unroll
+  for (int i = 0; i < NXF; i++) {
+    xlo[i] = ldv(&xloV[i]) + ldv(&xloC[i]);
+    xhi[i] = ldv(&xhiV[i]) + ldv(&xhiC[i]);
+  }
+#pragma unroll
+  for (int z = 0; z < TZ / 2; z++) corr[z] = ldv(&corrV[z]);
+  const float czc0 = ldv(&czc0V), czc1 = ldv(&czc1V);
   // the column into registers
   const int own = ty * TX + tx;
   float xr[TZ + 2], bb[TZ], rd[TZ], czr[TZ + 1];
