@@ -115,14 +115,24 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
     const int64_t c = base + ((int64_t)((lz << L) + ly) << L) + lx;
 
     // All loads as stored, the conversions after the last one (a conversion waits for its
-    // load); the x neighbours, which may need a block's table entry first, come last.
+    // load).  FP16: the x neighbours, which may need a block's table entry first, come last, and
+    // the right-hand side early; FP32 rows leave no registers for that.
+    constexpr bool H = sizeof(V) == 2;
     RawRow<V, CPT> xv, dv, cxv, cyv, czv, ym, yq, zm, zq, cyu, czu, bRow;
     xv.ld(x + c);
     dv.ld(d + c);
     cxv.ld(cx + c);
     cyv.ld(cy + c);
     czv.ld(cz + c);
-    if constexpr (MODE > 0) bRow.ld(b + c);
+    if constexpr (MODE > 0 && H) bRow.ld(b + c);
+    V xlV = V(0.f), xrV = V(0.f), cxrV = V(0.f);
+    auto xSides = [&]() {
+      const int64_t j = lx > 0 ? c - 1 : cellAt(g, s, lx - 1, ly, lz);
+      if (j >= 0) xlV = x[j];
+      const int64_t k = lx + CPT < bs ? c + CPT : cellAt(g, s, lx + CPT, ly, lz);
+      if (k >= 0) { xrV = x[k]; cxrV = cx[k]; }
+    };
+    if constexpr (!H) xSides();
     {
       const int64_t j = ly > 0 ? c - sy : cellAt(g, s, lx, ly - 1, lz);
       if (j >= 0) ym.ld(x + j); else ym.zero();
@@ -137,13 +147,7 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
       if (k >= 0) { zq.ld(x + k); czu.ld(cz + k); }
       else { zq.zero(); czu.zero(); }
     }
-    V xlV = V(0.f), xrV = V(0.f), cxrV = V(0.f);
-    {
-      const int64_t j = lx > 0 ? c - 1 : cellAt(g, s, lx - 1, ly, lz);
-      const int64_t k = lx + CPT < bs ? c + CPT : cellAt(g, s, lx + CPT, ly, lz);
-      if (j >= 0) xlV = x[j];
-      if (k >= 0) { xrV = x[k]; cxrV = cx[k]; }
-    }
+    if constexpr (H) xSides();
     const float xl = ldv(&xlV), xr = ldv(&xrV), cxr = ldv(&cxrV);
     float r[CPT];
     if constexpr (MODE == 2) {
@@ -151,6 +155,7 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
       // r = b - A x in double-float arithmetic: every product split exactly into
       // a rounded part and its error (fma), the running sum kept exact with
       // TwoSum and the errors gathered in a second float; then sum r^2, b^2.
+      if constexpr (!H) bRow.ld(b + c);
       float rq = 0.f, bq = 0.f;
 #pragma unroll
       for (int i = 0; i < CPT; i++) {
@@ -200,6 +205,7 @@ __global__ void __launch_bounds__(256, CPT == 4 || sizeof(V) == 2 ? 3 : 2)
       r[i] = a;
     }
     if constexpr (MODE == 1) {
+      if constexpr (!H) bRow.ld(b + c);
 #pragma unroll
       for (int i = 0; i < CPT; i++) r[i] = bRow[i] - r[i];
     }
