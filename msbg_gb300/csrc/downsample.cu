@@ -16,19 +16,21 @@
 // reference's four 4-wide accumulators (one per row, lanes = x offsets) and its
 // horizontal add.
 //
-// One CTA per value block, one thread per coarse (x, y) column, marching the
-// coarse planes in z.  Fine planes with their 1-cell x/y halo are staged as FP32
+// One CTA per value block, one thread per two coarse (x, y) columns (neighbours in y, which
+// share two of their fine rows), marching the coarse planes in z.  Fine planes with their 1-cell x/y halo are staged as FP32
 // in a 4-plane shared-memory ring ([bs+2][bs+2] each, rows coalesced along x), two
 // new planes per coarse plane, so each fine plane is read from memory once; the
 // loads of the next two planes are in flight while the current two are used.  Each
-// thread carries its 16 partial sums of the coarse plane above in registers.
+// thread carries the 32 partial sums of its cells of the coarse plane above in registers.
 // The planes in flight are kept as stored and widened when they are put into the ring:
 // a conversion at the load would wait for it.  The thread's ring cells are looked up
 // once for the block's own z-layer, the sums run in column pairs on the packed FP32
 // pipe (the same operations per column).  Floor: S bytes per fine cell read, 4 per
 // coarse cell written (236 M FP16 cells: 85 us); measured 322 us with per-plane lookups
-// and conversions at the load, 274 with the lookups and the pairs alone, 199 with all.
-// Bound now: the latency of a CTA's steps (64 registers, half the warps an SM holds).
+// and conversions at the load, 274 with the lookups and the pairs of columns alone, 199
+// with planes as stored, 193 with the rows' stores in different banks, 177 with two cells
+// a thread (six row reads for two cells where one takes four; the shared-memory pipe was
+// 84% busy).  Five CTAs a SM instead of four (96 registers): 180.
 #include "internal.cuh"
 
 namespace msbg {
@@ -54,7 +56,7 @@ __device__ __forceinline__ void quadVals(const uint2 &q, float v[4], const uint1
 
 template <int BS>
 constexpr int dsThreads() {
-  return (BS / 2) * (BS / 2) < 32 ? 32 : (BS / 2) * (BS / 2);
+  return BS / 2 * BS / 4 < 32 ? 32 : BS / 2 * BS / 4;
 }
 
 template <typename T, int BS, bool SIMPLE>
@@ -83,11 +85,10 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   // domain face), 4 consecutive values per thread; the ring of 4 (BS + 1) halo cells
   // goes cell by cell.  fetch issues the loads into registers, put stores them into
   // the ring slot.
-  constexpr int NI = BS * BS / 4, NR = 4 * (BS + 1), PR = (NR + NT - 1) / NT;
-  static_assert(NI <= NT, "one interior quad per thread");
+  constexpr int NI = BS * BS / 4, NR = 4 * (BS + 1), PR = (NR + NT - 1) / NT, PQ = (NI + NT - 1) / NT;
   // a plane's values as stored: a conversion here would wait for the loads it follows
   struct Plane {
-    typename Quad<T>::V in;
+    typename Quad<T>::V in[PQ];
     T ring[PR];
   };
   const T zero = T(0.0f);  // the empty value
@@ -117,7 +118,10 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   const T *quadSrc = pay + ((int64_t)t << (3 * L)) + 4 * tid;
   auto fetch = [&](int p, Plane &v) {
     if (p >= 0 && p < BS) {
-      if (tid < NI) v.in = *reinterpret_cast<const typename Quad<T>::V *>(quadSrc + (p << (2 * L)));
+#pragma unroll
+      for (int k = 0; k < PQ; k++)
+        if (tid + k * NT < NI)
+          v.in[k] = *reinterpret_cast<const typename Quad<T>::V *>(quadSrc + 4 * NT * k + (p << (2 * L)));
 #pragma unroll
       for (int k = 0; k < PR; k++)
         v.ring[k] = ringSrc[k] ? ringSrc[k][p << (2 * L)] : zero;
@@ -126,10 +130,12 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
     const int gz = min(max((bz << L) + p, 0), sz - 1);
     const int nz = ((gz >> L) - bz + 1) * 9 + 1;
     const int64_t zoff = (int64_t)(gz & m) << (2 * L);
-    if (tid < NI) {
-      const int sc = nbs[nz + 3];  // the block above / below (or the own block)
-      v.in = {};
-      if (sc >= 0) v.in = *reinterpret_cast<const typename Quad<T>::V *>(pay + ((int64_t)sc << (3 * L)) + zoff + 4 * tid);
+    const int sc = nbs[nz + 3];  // the block above / below (or the own block)
+#pragma unroll
+    for (int k = 0; k < PQ; k++) {
+      v.in[k] = {};
+      if (sc >= 0 && tid + k * NT < NI)
+        v.in[k] = *reinterpret_cast<const typename Quad<T>::V *>(pay + ((int64_t)sc << (3 * L)) + zoff + 4 * (tid + k * NT));
     }
 #pragma unroll
     for (int k = 0; k < PR; k++) {
@@ -146,20 +152,26 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   };
   auto put = [&](int p, const Plane &v) {
     float *dst = st + ((p + 1) & 3) * HH;
-    if (tid < NI) {
-      const int r = (4 * tid) >> L, c = (4 * tid) & m;
+#pragma unroll
+    for (int u = 0; u < PQ; u++) {
+      const int e = tid + u * NT;
+      if (e >= NI) break;
+      const int r = (4 * e) >> L, c = (4 * e) & m;
       float *q = dst + (r + 1) * H + c + 1;
       float in[4];
-      quadVals(v.in, in, (const T *)nullptr);
+      quadVals(v.in[u], in, (const T *)nullptr);
+      // 32-wide rows: two pairs of rows of a warp lie in the same banks for one k; the second
+      // pair stores its values in the order 1, 0, 3, 2
+      const int sw = BS == 32 ? (e >> 4) & 1 : 0;
 #pragma unroll
-      for (int k = 0; k < 4; k++) q[k] = in[k];
+      for (int k = 0; k < 4; k++) q[k ^ sw] = sw ? in[k ^ 1] : in[k];
     }
 #pragma unroll
     for (int k = 0; k < PR; k++)
       if (ringDst[k] >= 0) dst[ringDst[k]] = Store<T>::load(&v.ring[k]);
   };
-  const bool own = tid < CB * CB;
-  const int vx = tid & (CB - 1), vy = tid / CB;
+  const bool own = tid < CB * CB / 2;
+  const int vx = tid & (CB - 1), vy = 2 * (tid / CB);  // coarse cells (vx, vy) and (vx, vy + 1)
   // exact weights k1[k] k1[j] k1[i] / 512 of (plane k, row j, columns i = 2h, 2h + 1)
   auto wgt = [](int k, int j, int h) {
     const float k1[4] = {1.f, 3.f, 3.f, 1.f};
@@ -176,8 +188,8 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   // (2vz+1, 2vz+2) completes them (k = 2, 3) and starts those of plane vz+1.  The
   // next pair's loads are in flight while a pair is used.
   const float2 zero2 = make_float2(0.0f, 0.0f);
-  float2 acc[4][2];  // acc[j][h]: columns 2h, 2h + 1 over k = 0, 1
-  float part = 0.0f;  // part: the children sum in plane 2vz
+  float2 acc[2][4][2];  // [cell][j][h]: columns 2h, 2h + 1 over k = 0, 1
+  float part[2] = {0.0f, 0.0f};  // the children sums in plane 2vz
   // Fine-plane pairs go through two register sets (A: pairs of even coarse planes, B:
   // odd), so the loads of the next two pairs are in flight while a pair is used.
   Plane va, vb, vc, vd;
@@ -192,15 +204,20 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
   fetch(4, vd);
   if (own) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < 6; j++) {
       float2 r0[2], r1[2];
       row(-1, j, r0);
       row(0, j, r1);
 #pragma unroll
-      for (int h = 0; h < 2; h++)
-        if (!SIMPLE) acc[j][h] = __ffma2_rn(wgt(1, j, h), r1[h], __ffma2_rn(wgt(0, j, h), r0[h], zero2));
-      if (SIMPLE && j == 1) part = __fadd_rn(r1[0].y, r1[1].x);
-      if (SIMPLE && j == 2) part = __fadd_rn(__fadd_rn(part, r1[0].y), r1[1].x);
+      for (int y = 0; y < 2; y++) {
+        const int jy = j - 2 * y;  // row of cell vy + y
+        if (jy < 0 || jy > 3) continue;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          if (!SIMPLE) acc[y][jy][h] = __ffma2_rn(wgt(1, jy, h), r1[h], __ffma2_rn(wgt(0, jy, h), r0[h], zero2));
+        if (SIMPLE && jy == 1) part[y] = __fadd_rn(r1[0].y, r1[1].x);
+        if (SIMPLE && jy == 2) part[y] = __fadd_rn(__fadd_rn(part[y], r1[0].y), r1[1].x);
+      }
     }
   }
   // one coarse plane from the pair (p, q) of fine planes 2vz+1, 2vz+2
@@ -215,29 +232,36 @@ __global__ void __launch_bounds__(dsThreads<BS>(), 4) kDownsample(const T *__res
       fetch(2 * vz + 6, q);
     }
     if (!own) return;
-    float2 T2[2];
-    float sum = part, npart = 0.0f;
+    float2 T2[2][2];
+    float sum[2] = {part[0], part[1]};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < 6; j++) {
       float2 r2[2], r3[2];
       row(2 * vz + 1, j, r2);
       row(2 * vz + 2, j, r3);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        if (SIMPLE) break;
-        const float2 S = __ffma2_rn(wgt(3, j, h), r3[h], __ffma2_rn(wgt(2, j, h), r2[h], acc[j][h]));
-        T2[h] = j == 0 ? S : __fadd2_rn(T2[h], S);
-        acc[j][h] = __ffma2_rn(wgt(1, j, h), r3[h], __ffma2_rn(wgt(0, j, h), r2[h], zero2));
-      }
-      if (SIMPLE && (j == 1 || j == 2)) {  // children in plane 2vz+1 (this cell) and 2vz+2 (the next)
-        sum = __fadd_rn(__fadd_rn(sum, r2[0].y), r2[1].x);
-        npart = j == 1 ? __fadd_rn(r3[0].y, r3[1].x) : __fadd_rn(__fadd_rn(npart, r3[0].y), r3[1].x);
+      for (int y = 0; y < 2; y++) {
+        const int jy = j - 2 * y;
+        if (jy < 0 || jy > 3) continue;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          if (SIMPLE) break;
+          const float2 S = __ffma2_rn(wgt(3, jy, h), r3[h], __ffma2_rn(wgt(2, jy, h), r2[h], acc[y][jy][h]));
+          T2[y][h] = jy == 0 ? S : __fadd2_rn(T2[y][h], S);
+          acc[y][jy][h] = __ffma2_rn(wgt(1, jy, h), r3[h], __ffma2_rn(wgt(0, jy, h), r2[h], zero2));
+        }
+        if (SIMPLE && (jy == 1 || jy == 2)) {  // children in plane 2vz+1 (this cell) and 2vz+2 (the next)
+          sum[y] = __fadd_rn(__fadd_rn(sum[y], r2[0].y), r2[1].x);
+          part[y] = jy == 1 ? __fadd_rn(r3[0].y, r3[1].x) : __fadd_rn(__fadd_rn(part[y], r3[0].y), r3[1].x);
+        }
       }
     }
-    part = npart;
-    const float val = SIMPLE ? __fmul_rn(sum, 0.125f)
-                             : __fadd_rn(__fadd_rn(T2[0].x, T2[0].y), __fadd_rn(T2[1].x, T2[1].y));
-    out[(int64_t)t * CB * CB * CB + ((int64_t)vz * CB + vy) * CB + vx] = val;
+#pragma unroll
+    for (int y = 0; y < 2; y++) {
+      const float val = SIMPLE ? __fmul_rn(sum[y], 0.125f)
+                               : __fadd_rn(__fadd_rn(T2[y][0].x, T2[y][0].y), __fadd_rn(T2[y][1].x, T2[y][1].y));
+      out[(int64_t)t * CB * CB * CB + ((int64_t)vz * CB + vy + y) * CB + vx] = val;
+    }
   };
   static_assert(CB % 2 == 0, "coarse planes in pairs");
 #pragma unroll 1
