@@ -567,7 +567,7 @@ def halo_measure(g, info, storage, elem, bsx, steps, dist, peaks, bound: list, b
     d_bids.free()
     nbytes = len(bids) * hs ** 3 * (elem + 4)
     gbs = nbytes / (ms / 1e3) / 1e9
-    return {"kernel": "kFillHalo (OPT_BC_COARSE_LEVEL, halo 1)", "blocks": int(len(bids)),
+    return {"kernel": "kFillHaloRows (OPT_BC_COARSE_LEVEL, halo 1)", "blocks": int(len(bids)),
             "level1_blocks": n1, "ms_per_pass": ms, "blocks_per_s": len(bids) * dist.world / (ms / 1e3),
             "launches_per_pass": int(launches), "skipped": int(sk),
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
@@ -650,11 +650,11 @@ def render_measure(g, steps, dist, cpu: bool, width=1920, height=1080) -> dict:
     g._check(g.L.msbg_gpu_copy_d2h(g.h, G._ptr(img), C.c_void_p(d_rgb.ptr), img.nbytes))
     g.synchronize()
     d_rgb.free()
-    out = {"kernel": "kRender (FP64 ray march, cubic B-spline normal)", "width": width, "height": height,
+    out = {"kernel": "kRender (ray march on FP64 positions stepped as integers, cubic B-spline normal)", "width": width, "height": height,
            "camera": "demo (src/msbg_demo.cpp:123-127)", "ms_per_frame": ms,
            "pixels_per_s": width * height * dist.world / (ms / 1e3), "hit_pixels": int(img.any(-1).sum()),
            "launches_per_frame": (g.launch_count() - l0) // n,
-           "bound": "FP64 pipe (3 adds + 3 conversions per ray step) and gathers near the surface"}
+           "bound": "issue, and gathers near the surface"}
     if cpu:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import port as P  # the oracle, as the CPU baseline
