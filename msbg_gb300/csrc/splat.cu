@@ -87,7 +87,7 @@ __device__ __forceinline__ bool splatBox(const SplatGeom &g, float px, float py,
 // come one after another, so thousands of atomics at a time met on the same few hundred
 // addresses (2.05 M particles of the 512^3 workload: 346 us to count, 357 us to scatter).
 // A CTA therefore sums its particles' blocks in a hash table in shared memory and goes to
-// the global counters once per block (@LISTS@).  A block that finds no place within
+// the global counters once per block (33 and 62 us).  A block that finds no place within
 // kHashProbes goes to the global counter directly; whether it has a place is the same for
 // every thread and both passes over the particles, since places are never given back.
 constexpr int kListThreads = 512, kHashSize = 2048, kHashProbes = 16;
