@@ -133,8 +133,8 @@ struct ColorArgs {
 // The fast 7-point form: a thread needs its own four voxels of the planes z=-1 and z=BS, which
 // it reads from global memory, and no corner.  Without those pieces (4.9 KB) three CTAs of a
 // 32^3 block share an SM (72 registers): FP16, 514 M voxels, 10 iterations, 6.12 -> 4.92 ms.
-// The same for MCF (80 registers, planes from global memory) was slower on 102 M voxels, 2.51 ->
-// 2.66 ms.
+// The same for MCF (80 registers, planes from global memory) was slower at every size: 216 / 512 /
+// 4096 blocks a pass 19.7 -> 26.6, 38.2 -> 45.5, 241 -> 252 us.
 template <typename T, int FK>
 constexpr bool facesOnly() { return sizeof(T) == 2 && (FK & ~FK_CLAMP) == K_JACOBI; }
 
