@@ -15,12 +15,23 @@
 // Autotuning: the grid of the per-block dot kernel and of the vector updates (CTAs
 // per SM) is chosen once per layout by timing the candidates on the live data.
 #include <algorithm>
+#include <tuple>
 #include <vector>
 
 #include "internal.cuh"
 #include "poisson.cuh"
 
 namespace msbg {
+
+// What the captured iteration holds by value and a later call can change: the solution, the
+// right-hand side, the tolerance and the V-cycle's parameters and coarsest solve.  (The work
+// vectors go with poisson_release_work, which drops the graph; all else lives as long as the
+// layout, and so does the graph.)
+using GraphKey = std::tuple<const void *, const void *, double, int, int, int, int, const void *, bool>;
+static GraphKey graphKeyOf(const PoissonState *ps, const float *x, const float *b, double tol) {
+  return GraphKey(x, b, tol, ps->preSweeps, ps->postSweeps, ps->tileIters, ps->coarsestIter, ps->dCoarseInv,
+                  ps->coarseInvValid);
+}
 
 struct BatchState {
   int64_t layoutStamp = -1;
@@ -36,8 +47,7 @@ struct BatchState {
   int updGrid = 0;               // autotuned grid of the vector kernels
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
-  const void *graphKey[3] = {};  // x, b, tol bits of the captured iteration
-  double graphTol = 0.0;
+  GraphKey graphKey;  // of the captured iteration
 };
 
 // rows of the per-volume scalar array
@@ -175,6 +185,12 @@ void batchFree(BatchState *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
+}
+
+void batchDropGraph(BatchState *b) {
+  if (!b || !b->graph) return;
+  cudaGraphExecDestroy(b->graph);
+  b->graph = nullptr;
 }
 
 // Host-side declarations of the Poisson pieces used here (poisson.cu)
@@ -357,7 +373,8 @@ extern "C" int msbg_gpu_batch_mgpcg_solve(msbg_gpu_ctx *ctx, int chanX, int chan
   MSBG_CUDA(ctx, cudaMemcpyAsync(p, z, (size_t)n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
   if ((rc = segDot(ctx, bs, r, z, bs->vs + kVsRz * nV))) return rc;
 
-  const bool graphOk = useGraph && bs->graph && bs->graphKey[0] == x && bs->graphKey[1] == b && bs->graphTol == tol;
+  const GraphKey key = graphKeyOf(ps, x, b, tol);
+  const bool graphOk = useGraph && bs->graph && bs->graphKey == key;
   int it = 1;
   // iterations it, it+1, ... until every volume has met the tolerance on its
   // recurrence residual (it is then the last iteration run) or maxIter has run
@@ -375,7 +392,7 @@ extern "C" int msbg_gpu_batch_mgpcg_solve(msbg_gpu_ctx *ctx, int chanX, int chan
         MSBG_CUDA(ctx, cudaGraphInstantiate(&bs->graph, gr, 0));
         cudaGraphDestroy(gr);
         ctx->launches = l0;  // captured, not launched
-        bs->graphKey[0] = x; bs->graphKey[1] = b; bs->graphTol = tol;
+        bs->graphKey = key;
       }
       if (useGraph && bs->graph && (graphOk || it >= 2)) {
         MSBG_CUDA(ctx, cudaGraphLaunch(bs->graph, ctx->stream));

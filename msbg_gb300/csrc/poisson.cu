@@ -831,6 +831,7 @@ extern "C" int msbg_gpu_poisson_release_work(msbg_gpu_ctx *ctx) {
   if (!ctx) return MSBG_GPU_ERR_ARG;
   if (!ctx->poisson) return MSBG_GPU_OK;
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  batchDropGraph(ctx->batch);  // its kernels work on the vectors freed here
   for (PrecSet *P : {&ctx->poisson->f32, &ctx->poisson->f16}) {
     for (void **q : {&P->vr, &P->vp, &P->vz, &P->vs, &P->ve, &P->vb}) {
       if (*q) cudaFree(*q);
