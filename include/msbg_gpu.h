@@ -326,7 +326,9 @@ int msbg_gpu_set_relax_params(msbg_gpu_ctx *ctx, float omega, int blockIter);
 /* Diagnostics of the failure path: one CTA waits on an mbarrier that nothing completes,
  * with the same bounded try-wait loop as the library's kernels but a limit of `polls`
  * (1..1<<20).  The kernel records the expired wait in the device status word and returns;
- * the call returns MSBG_GPU_ERR_TIMEOUT, clears the word, and leaves the context usable.
+ * the call returns MSBG_GPU_ERR_TIMEOUT, clears the word, and leaves the context usable
+ * (and the V-cycle's grid barrier with a count that an expired wait can leave: the next
+ * cycle does not depend on it).
  * No GPU fault is involved. */
 int msbg_gpu_diag_wait_timeout(msbg_gpu_ctx *ctx, int polls);
 /* downsampleFloatChannelNew (src/msbg4.cpp:1035-1379, levelMg = 1, OPT_ALL_CELLS): the

@@ -455,7 +455,6 @@ extern "C" int msbg_gpu_batch_mgpcg_solve(msbg_gpu_ctx *ctx, int chanX, int chan
   MSBG_CUDA(ctx, cudaMemcpy(&st, ctx->dStatus, sizeof(int), cudaMemcpyDeviceToHost));
   if (st) {
     MSBG_CUDA(ctx, cudaMemset(ctx->dStatus, 0, sizeof(int)));
-    if (ps->dTailBar) MSBG_CUDA(ctx, cudaMemset(ps->dTailBar, 0, 2 * sizeof(unsigned)));
     return fail(ctx, MSBG_GPU_ERR_TIMEOUT, "a bounded device wait timed out (status bits %d)", st);
   }
   return MSBG_GPU_OK;

@@ -1161,6 +1161,7 @@ extern "C" int msbg_gpu_diag_wait_timeout(msbg_gpu_ctx *ctx, int polls) {
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st) {
     MSBG_CUDA(ctx, cudaMemsetAsync(ctx->dStatus, 0, sizeof(int), ctx->stream));
+    if (const int rc = tailCounterGaveUp(ctx)) return rc;
     MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return fail(ctx, MSBG_GPU_ERR_TIMEOUT, "a bounded device wait timed out (status bits %d)", st);
   }

@@ -22,6 +22,8 @@ void levelChannelsFree(LevelChannels *lc);
 void warmNetFree(WarmNetState *w);
 void batchFree(BatchState *b);
 void batchDropGraph(BatchState *b);
+// Diagnostics: the counter of the small levels' barrier as a wait that gave up leaves it.
+int tailCounterGaveUp(msbg_gpu_ctx *ctx);
 constexpr int kMaxChannels = 64;
 // device counters of a context (int64): 0 nActParticles, 1 nAborted, 2 nActive,
 // 3 scratch, 4..11 blocks per level (5, 6 reused as scan totals by the solver),

@@ -810,11 +810,17 @@ static int checkStatus(msbg_gpu_ctx *ctx) {
   MSBG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st) {
     MSBG_CUDA(ctx, cudaMemsetAsync(ctx->dStatus, 0, sizeof(int), ctx->stream));
-    if (ctx->poisson && ctx->poisson->dTailBar)
-      MSBG_CUDA(ctx, cudaMemsetAsync(ctx->poisson->dTailBar, 0, 2 * sizeof(unsigned), ctx->stream));
     return fail(ctx, MSBG_GPU_ERR_TIMEOUT, "a bounded device wait timed out (status bits %d)", st);
   }
   return MSBG_GPU_OK;
+}
+
+// What a solve that diverged returns: the device wait that gave up, if one did (a V-cycle it
+// cut short gives such residuals), and then no later call finds the status bits.
+static int divergedOrTimeout(msbg_gpu_ctx *ctx, int rc) {
+  if (rc != MSBG_GPU_ERR_DIVERGED) return rc;
+  const int st = checkStatus(ctx);
+  return st ? st : rc;
 }
 
 // The level-0 FP32 work vectors r, p, z, s of the FP32 solves (4 x 4 B per cell).
@@ -1112,7 +1118,8 @@ extern "C" int msbg_gpu_mgpcg_solve(msbg_gpu_ctx *ctx, int chanX, int chanB, dou
   double rel = bnorm > 0 ? sqrt(rr0) / bnorm : 0.0;
   int it = 0;
   if (bnorm > 0 && rel > tol) {
-    if ((rc = pcgT<float>(ctx, ps, ps->f32, x, b, r, tol * bnorm, maxIter, true, bnorm, &it, &rel))) return rc;
+    if ((rc = pcgT<float>(ctx, ps, ps->f32, x, b, r, tol * bnorm, maxIter, true, bnorm, &it, &rel)))
+      return divergedOrTimeout(ctx, rc);
   }
   if (itersOut) *itersOut = it;
   if (relResOut) *relResOut = rel;
@@ -1148,7 +1155,7 @@ extern "C" int msbg_gpu_mgpcg_solve_mixed(msbg_gpu_ctx *ctx, int chanX, int chan
       return rc;
     if ((rc = fetchScal(ctx, ps, 8, 2))) return rc;
     const double rr = ps->hScal[8], bb = ps->hScal[9];
-    if (!isfinite(rr)) return fail(ctx, MSBG_GPU_ERR_DIVERGED, "outer residual not finite");
+    if (!isfinite(rr)) return divergedOrTimeout(ctx, fail(ctx, MSBG_GPU_ERR_DIVERGED, "outer residual not finite"));
     const double bnorm = sqrt(bb);
     rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
     if (bnorm == 0.0 || rel <= tol || outer >= maxOuter) break;
@@ -1164,7 +1171,7 @@ extern "C" int msbg_gpu_mgpcg_solve_mixed(msbg_gpu_ctx *ctx, int chanX, int chan
     int itIn = 0;
     double relIn = 0.0;
     if ((rc = pcgT<__half>(ctx, ps, ps->f16, e, rw, rw, innerTol * rhn, maxInner, false, rhn, &itIn, &relIn)))
-      return rc;
+      return divergedOrTimeout(ctx, rc);
     innerTotal += itIn;
     eScale = 1.0f / invScale;
     haveE = true;

@@ -42,7 +42,7 @@ struct TailArgs {
   int n, firstSmall;  // levels; the first that CTA 0 runs alone
   int npre, npost;    // red-black sweeps before and after the coarser level
   const float *inv;   // inverse of the coarsest operator
-  unsigned *bar;      // [0] arrivals, [1] CTAs done; zero between launches
+  unsigned *bar;      // arrivals; zero at the launch
   int *status;
 };
 
@@ -281,10 +281,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) kCoarseTail(const __grid_cons
     if (!sync()) break;
     smooth<V, false>(a.lv[l], x, a.npost, true, false, t0, stride, sync);
   }
-  if (threadIdx.x == 0) {
-    if (!ok) atomicOr(a.status, 32);  // the host zeroes the counters then
-    else if (atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) { a.bar[0] = 0; a.bar[1] = 0; }  // every CTA is past its barriers
-  }
+  if (!ok && threadIdx.x == 0) atomicOr(a.status, 32);
 }
 
 // parent of every cell of the finer level (blocks of one cell), children of every coarse one
@@ -303,8 +300,7 @@ __global__ void kParentChild(const int32_t *__restrict__ activeF, int64_t n, int
 }  // namespace
 
 int tailBuildTables(msbg_gpu_ctx *ctx, PoissonState *ps) {
-  MSBG_CUDA(ctx, cudaMalloc(&ps->dTailBar, 2 * sizeof(unsigned)));
-  MSBG_CUDA(ctx, cudaMemsetAsync(ps->dTailBar, 0, 2 * sizeof(unsigned), ctx->stream));
+  MSBG_CUDA(ctx, cudaMalloc(&ps->dTailBar, sizeof(unsigned)));
   for (size_t l = 1; l < ps->levels.size(); l++) {
     MgLevel &F = ps->levels[l - 1], &C = ps->levels[l];
     if (C.sameSet) continue;
@@ -363,11 +359,20 @@ int coarseTail(msbg_gpu_ctx *ctx, PoissonState *ps, const PrecSet &P, size_t l, 
   int64_t grid = (a.lv[0].nCell / 2 + kTailThreads - 1) / kTailThreads;
   if (grid > nSm) grid = nSm;
   if (grid < 1 || a.firstSmall == 0) grid = 1;
+  // The counter starts at zero for every launch: one that a kernel's last CTA had reset stayed
+  // as it was when a wait gave up, and the next launch's phases would not have been separated.
+  MSBG_CUDA(ctx, cudaMemsetAsync(ps->dTailBar, 0, sizeof(unsigned), ctx->stream));
   void *args[] = {&a};
   MSBG_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kCoarseTail<V>, dim3((unsigned)grid), dim3(kTailThreads), args, 0,
                                              ctx->stream));
   ctx->launches++;
   *done = true;
+  return MSBG_GPU_OK;
+}
+
+int tailCounterGaveUp(msbg_gpu_ctx *ctx) {
+  if (ctx->poisson && ctx->poisson->dTailBar)
+    MSBG_CUDA(ctx, cudaMemsetAsync(ctx->poisson->dTailBar, 0x01, sizeof(unsigned), ctx->stream));
   return MSBG_GPU_OK;
 }
 
