@@ -392,7 +392,8 @@ enum { MSBG_GPU_LBLK_EMPTY = -1, MSBG_GPU_LBLK_FULL = -2, MSBG_GPU_LBLK_NONE = -
 int msbg_gpu_level_grid_set(msbg_gpu_ctx *ctx, int lchan, int level, int storage, const int32_t *hState,
                             const void *hPayload, int64_t nData, float emptyValue, float fullValue);
 /* The same for data already on the device: binds the caller's device arrays (dState:
- * nBlocks states; dPayload: the payload blocks, 16-byte aligned) without copying.  They
+ * nBlocks states; dPayload: the payload blocks, aligned to their elements; 16-byte aligned
+ * ones are read in vectors) without copying.  They
  * must stay valid, and unchanged while a fill reads them, until the level is set or
  * bound again or the context is destroyed.  A level-0 value-block channel binds as its slab
  * (msbg_gpu_payload_ptr) with states = its slots, -3 for blocks that are not at level 0. */

@@ -82,7 +82,7 @@ struct HaloArgs {
   int sx, sy, sz;         // level-l domain
   int nbx, nby, nbz;
   int opt;
-  int quadOk, pairOk;     // kFillHaloRows: level l (l+1) payload aligned to 4 (2) elements
+  int quadOk, pairOk;     // level l payload aligned to 4 elements, level l+1 payload to 2
   float *out;
   unsigned long long *skipped;
 };
@@ -222,9 +222,16 @@ __global__ void __launch_bounds__(kHaloThreads, 8) kFillHalo(HaloArgs a) {
     } else {
       for (int k = threadIdx.x; k < bs * bs / 4; k += kHaloThreads) {
         const int xq = k & ((bs >> 2) - 1), y = k >> (L - 2);
+        const T *q = blk + (z * bs + y) * bs + 4 * xq;
         float v[4];
-        if (blk) load4<T>(blk + (z * bs + y) * bs + 4 * xq, v);
-        else v[0] = v[1] = v[2] = v[3] = cOwn;
+        if (!blk) {
+          v[0] = v[1] = v[2] = v[3] = cOwn;
+        } else if (a.quadOk) {
+          load4<T>(q, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[i] = ldRaw<T>(q + i);
+        }
         float *o = buf + (y + h) * hs + h + 4 * xq;
         o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; o[3] = v[3];
       }
@@ -536,7 +543,8 @@ float quantConst(int storage, float v) {
 // them, beside bs quads); other boxes go plane by plane.
 template <typename T>
 int fillHaloLaunch(msbg_gpu_ctx *ctx, HaloArgs a, int64_t n, size_t smem) {
-  // caller arrays may be aligned to their elements only
+  // Caller arrays may be aligned to their elements only: rows are then read one by one, in
+  // either form.
   a.quadOk = ((uintptr_t)a.lv.pay & (4 * sizeof(T) - 1)) == 0;
   a.pairOk = ((uintptr_t)a.lo.pay & (2 * sizeof(T) - 1)) == 0;
   const size_t rows = (size_t)(kHaloRowThreads / 32) * (a.bs >= 8 ? 32 / a.bs : 0) * 4 * a.hs * sizeof(float);
