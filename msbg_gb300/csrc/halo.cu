@@ -193,7 +193,9 @@ __global__ void __launch_bounds__(kHaloThreads, 8) kFillHalo(HaloArgs a) {
     return src.p ? ldRaw<T>(src.p) : src.c;
   };
   const int L = a.log2bs;
-  if (bs < 4) {  // every position the general way
+  // Every position the general way where rows are no vectors (a choice between loads in the
+  // loop below cost aligned payloads 4 to 6%).
+  if (bs < 4 || !a.quadOk) {
     for (int i = threadIdx.x; i < per; i += kHaloThreads) {
       const int q = (int)__umulhi((uint32_t)i, a.hsMagic), hz = (int)__umulhi((uint32_t)q, a.hsMagic);
       dst[i] = value(i - q * hs, q - hz * hs, hz);
@@ -222,16 +224,9 @@ __global__ void __launch_bounds__(kHaloThreads, 8) kFillHalo(HaloArgs a) {
     } else {
       for (int k = threadIdx.x; k < bs * bs / 4; k += kHaloThreads) {
         const int xq = k & ((bs >> 2) - 1), y = k >> (L - 2);
-        const T *q = blk + (z * bs + y) * bs + 4 * xq;
         float v[4];
-        if (!blk) {
-          v[0] = v[1] = v[2] = v[3] = cOwn;
-        } else if (a.quadOk) {
-          load4<T>(q, v);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; i++) v[i] = ldRaw<T>(q + i);
-        }
+        if (blk) load4<T>(blk + (z * bs + y) * bs + 4 * xq, v);
+        else v[0] = v[1] = v[2] = v[3] = cOwn;
         float *o = buf + (y + h) * hs + h + 4 * xq;
         o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; o[3] = v[3];
       }
