@@ -1309,11 +1309,8 @@ template <int BS>
 int launchRelaxMultires(msbg_gpu_ctx *ctx, const MrArgs &a, unsigned n, int parity, float omega, int blockIter,
                         int reverse, int countOutOfRange) {
   constexpr int smem = (BS + 2) * (BS + 2) * (BS + 2) * (int)sizeof(float);
-  static bool attr = false;
-  if (!attr) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kRelaxMultires<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  static SmemOptIn optIn;
+  MSBG_CUDA(ctx, optIn((const void *)kRelaxMultires<BS>, smem));
   MSBG_LAUNCH(ctx, kRelaxMultires<BS>, n, kMrThreads, smem, a, parity, omega, blockIter, reverse, countOutOfRange);
   return MSBG_GPU_OK;
 }

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "msbg_gpu.h"
+#include "smem_optin.h"
 
 namespace msbg {
 

@@ -1049,13 +1049,8 @@ static int smoothLaunch(msbg_gpu_ctx *ctx, PoissonState *ps, const MgLevel &Lv, 
   using Sh = TileShape<BS>;
   constexpr int NT = Sh::NT;
   constexpr size_t smem = tileSmemBytes<V, BS>();
-  static bool attrSet[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attrSet[dev]) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kTileSmooth<V, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attrSet[dev] = true;
-  }
+  static SmemOptIn optIn;
+  MSBG_CUDA(ctx, optIn((const void *)kTileSmooth<V, BS>, (int)smem));
   const int64_t nUnits = BS == 32 ? Lv.nAct * 4 : (tc == 0 ? ps->nEven : Lv.nAct - ps->nEven);
   if (nUnits <= 0) return MSBG_GPU_OK;
   constexpr int E = (int)sizeof(V);

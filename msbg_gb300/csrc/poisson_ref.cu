@@ -273,11 +273,8 @@ int launchRelaxRef(msbg_gpu_ctx *ctx, const int32_t *slots, int64_t n, BlkGeom g
                    const PrecSet &P, float omega, int blockIter, int reverse) {
   if (n <= 0) return MSBG_GPU_OK;
   constexpr size_t smem = sizeof(float) * (BS + 2) * (BS + 2) * (BS + 2);
-  static bool attr = false;
-  if (!attr) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kRelaxRef<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static SmemOptIn optIn;
+  MSBG_CUDA(ctx, optIn((const void *)kRelaxRef<BS>, (int)smem));
   MSBG_LAUNCH(ctx, kRelaxRef<BS>, (unsigned)n, kListThreads, smem, slots, g, x, b, (const float *)P.cx[0],
               (const float *)P.cy[0], (const float *)P.cz[0], (const float *)P.d[0], omega, blockIter, reverse);
   return MSBG_GPU_OK;

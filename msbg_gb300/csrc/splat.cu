@@ -534,11 +534,10 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
     const float *init = c.storage == MSBG_GPU_F32 ? dst : nullptr;
     auto blocks = [&](auto bsC, auto nzC) -> int {
       constexpr int BS = decltype(bsC)::value, NZ = decltype(nzC)::value, smem = splatSmemWords<BS, NZ>() * 4;
-      static bool attr = false;
-      if (smem > 48 * 1024 && !attr) {
-        MSBG_CUDA(ctx, cudaFuncSetAttribute(kSplatBlock<BS, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        MSBG_CUDA(ctx, cudaFuncSetAttribute(kSplatRest<BS, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
+      if (smem > 48 * 1024) {
+        static SmemOptIn optInBlock, optInRest;
+        MSBG_CUDA(ctx, optInBlock((const void *)kSplatBlock<BS, NZ>, smem));
+        MSBG_CUDA(ctx, optInRest((const void *)kSplatRest<BS, NZ>, smem));
       }
       MSBG_LAUNCH(ctx, (kSplatBlock<BS, NZ>), (unsigned)(NZ * nAct), splatThreads<BS>(), smem, dPts, g, ctx->dActive,
                   abortAt, off, entries, init, dst, nRest, rest);

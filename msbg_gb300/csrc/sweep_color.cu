@@ -597,12 +597,9 @@ template <typename T, int BS, int FK, int ZG>
 static cudaError_t launchPassT(const ColorArgs &a, unsigned blocks, cudaStream_t st) {
   const auto kern = kSweepColor<T, BS, FK, ZG>;
   constexpr size_t smem = colorSmemBytes<T, BS, FK>();
-  static bool attrSet = false;
-  if (!attrSet) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attrSet = true;
-  }
+  static SmemOptIn optIn;
+  const cudaError_t e = optIn((const void *)kern, (int)smem);
+  if (e != cudaSuccess) return e;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;

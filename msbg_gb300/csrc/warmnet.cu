@@ -1186,16 +1186,10 @@ static WnGeom wnGeom(const PoissonState *ps, const WarmNetState *w) {
 template <int BS1>
 static int wnConvStaged(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g) {
   constexpr size_t smem = stSmemBytes<BS1>();
-  static bool attr = false;
-  if (!attr) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kConvTcStaged<BS1, 2, 16, true, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kConvTcStaged<BS1, 16, 16, true, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kConvTcStaged<BS1, 16, 2, false, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static SmemOptIn optInFirst, optInMid, optInLast;
+  MSBG_CUDA(ctx, optInFirst((const void *)kConvTcStaged<BS1, 2, 16, true, true>, (int)smem));
+  MSBG_CUDA(ctx, optInMid((const void *)kConvTcStaged<BS1, 16, 16, true, false>, (int)smem));
+  MSBG_CUDA(ctx, optInLast((const void *)kConvTcStaged<BS1, 16, 2, false, false>, (int)smem));
   // resident CTAs per SM: 3 with the 58.5 KB of edge 16, 2 with the 87.5 KB of edge 8
   const unsigned gt = wnTcGrid(w->n1, smem <= 75 * 1024 ? 3 : 2);
   MSBG_LAUNCH(ctx, (kConvTcStaged<BS1, 2, 16, true, true>), gt, kTcThreads, smem, g, w->act[0], w->wq[0],
@@ -1242,12 +1236,8 @@ static int wnForward(msbg_gpu_ctx *ctx, const float *b0, float *x0) {
 template <int BS1, int CIN, int COUT, bool NORM>
 static int wnBwdWeight(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g, int l, const float *gp) {
   using W = BwdWeight<BS1, CIN, COUT>;
-  static bool attr = false;
-  if (!attr) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kBwdWeight<BS1, CIN, COUT, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)W::smem));
-    attr = true;
-  }
+  static SmemOptIn optIn;
+  MSBG_CUDA(ctx, optIn((const void *)kBwdWeight<BS1, CIN, COUT, NORM>, (int)W::smem));
   const int64_t nTiles = w->n1 / 512;
   const int grid = (int)(nTiles < kBwdParts ? nTiles : kBwdParts);
   MSBG_LAUNCH(ctx, (kBwdWeight<BS1, CIN, COUT, NORM>), (unsigned)grid, kBwdWThreads, W::smem, g, w->act[l], gp, w->dScal,
@@ -1260,11 +1250,8 @@ static int wnBwdWeight(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g, int 
 template <int BS1, int COUT>
 static int wnBwdData(msbg_gpu_ctx *ctx, WarmNetState *w, const WnGeom &g, int l, const float *gp, float *gx) {
   constexpr size_t smem = bwdDataSmem<BS1, COUT>();
-  static bool attr = false;
-  if (!attr) {
-    MSBG_CUDA(ctx, cudaFuncSetAttribute(kBwdData<BS1, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static SmemOptIn optIn;
+  MSBG_CUDA(ctx, optIn((const void *)kBwdData<BS1, COUT>, (int)smem));
   MSBG_LAUNCH(ctx, (kBwdData<BS1, COUT>), (unsigned)(w->n1 / 512), 256, smem, g, gp, w->act[l], w->wq[l], gx);
   return MSBG_GPU_OK;
 }
