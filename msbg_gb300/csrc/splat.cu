@@ -14,6 +14,7 @@
 // FP32 staging slab and the finalize quantizes the minimum to the storage type
 // first: rounding is monotonic, so quantize(min) == min(quantize) and the result
 // equals the demo's min over quantized values (src/msbg_demo.cpp:624-628).
+#include <algorithm>
 #include <type_traits>
 
 #include "internal.cuh"
@@ -90,11 +91,17 @@ __device__ __forceinline__ bool splatBox(const SplatGeom &g, float px, float py,
 // the global counters once per block (33 and 62 us).  A block that finds no place within
 // kHashProbes goes to the global counter directly; whether it has a place is the same for
 // every thread and both passes over the particles, since places are never given back.
+// Once half the places are taken, the CTA goes on without the table: most of its blocks come
+// once (particles in no order, or spread over a volume).
 constexpr int kListThreads = 512, kHashSize = 2048, kHashProbes = 16;
+constexpr int kDirectThreads = 256;  // of the forms without the table
 struct BlockHash {
   int key[kHashSize], val[kHashSize];
+  int taken, full;
+  __device__ __forceinline__ bool isFull() const { return *(const volatile int *)&full; }
 };
 __device__ __forceinline__ void hashClear(BlockHash &h) {
+  if (threadIdx.x == 0) h.taken = h.full = 0;
   for (int i = threadIdx.x; i < kHashSize; i += kListThreads) { h.key[i] = -1; h.val[i] = 0; }
 }
 // place of slot sl, claimed if INSERT; -1: none
@@ -106,7 +113,10 @@ __device__ __forceinline__ int hashPlace(BlockHash &h, int sl) {
     int at = *(volatile int *)&h.key[p];
     if (INSERT && at == -1) {
       at = atomicCAS(&h.key[p], -1, sl);
-      if (at == -1) return (int)p;
+      if (at == -1) {
+        if (atomicAdd(&h.taken, 1) >= kHashSize / 2) h.full = 1;
+        return (int)p;
+      }
     }
     if (at == sl) return (int)p;
     if (!INSERT && at == -1) return -1;
@@ -133,25 +143,47 @@ __device__ __forceinline__ bool boxSlots(const SplatGeom &g, const SplatBox &b, 
   return allValue;
 }
 
+// List entries that a CTA of the third pass takes: an eighth of an even share of all entries
+// over the CTAs that the chip holds (places), and at least 32 bs: without the share, 3 M
+// particles in no order split every list in two (32^3 blocks, radius 4: 2.99 ms, 2.37 so).
+// With fewer entries than two such chunks a place, four times that: a split list's chunks wait
+// for the first ones of all, which pays only where the blocks leave most places empty (100 k
+// particles in a ball, 32^3 blocks, 32 bs / four times that: radius 4 220 / 175 us, radius 10
+// 1085 / 907; the 64^3 frame's 38 blocks 1223 us a frame with four times that, 1183 so).
+struct ChunkRule {
+  int least, places, nz;
+  bool fewBlocks;
+  __host__ __device__ int of(int64_t total) const {
+    const int64_t share = total * nz / places;
+    if (share < 2 * least) return fewBlocks ? least : 4 * least;
+    return share / 8 < least ? least : (int)(share / 8);
+  }
+  int leastOf(int64_t upTo) const { return upTo * nz / places < 2 * least ? of(0) : least; }  // of any total
+};
+
 // Pass 1.  Valid particles (the marking loop's domain tests, src/msbg_demo.cpp:358-360, and
 // an owning value block: the demo walks the particle lists of value blocks only,
 // src/msbg_demo.cpp:541-566) get their abort index: the scan position (z, y, x order over
 // the box) of the first in-sphere voxel whose block is not a value block
 // (src/msbg_demo.cpp:613-618), or the box size.  Voxels from that position on are not
 // written.  Every value block the box touches counts the particle once.  abortAt = 0 marks
-// a particle that writes nothing.  A thread takes ppt particles, kListThreads apart.
-__global__ void __launch_bounds__(kListThreads) kSplatCount(const float *__restrict__ pts, int64_t n, int ppt, SplatGeom g,
+// a particle that writes nothing.  A thread takes ppt particles, NT apart; HASH: counted through
+// the table.
+template <int NT, bool HASH>
+__global__ void __launch_bounds__(NT) kSplatCount(const float *__restrict__ pts, int64_t n, int ppt, SplatGeom g,
                                                             const int32_t *__restrict__ slot,
                                                             int32_t *__restrict__ abortAt, int32_t *__restrict__ cnt,
                                                             unsigned long long *__restrict__ nAborted) {
   __shared__ BlockHash h;
-  hashClear(h);
-  __syncthreads();
+  if (HASH) {
+    hashClear(h);
+    __syncthreads();
+  }
   const int s = g.log2bs;
   const int64_t nxy = (int64_t)g.nbx * g.nby;
-  const int64_t first = (int64_t)blockIdx.x * ppt * kListThreads + threadIdx.x;
+  const int64_t first = (int64_t)blockIdx.x * ppt * NT + threadIdx.x;
   for (int q = 0; q < ppt; q++) {
-    const int64_t i = first + (int64_t)q * kListThreads;
+    const int64_t i = first + (int64_t)q * NT;
     if (i >= n) break;
     const float px = pts[3 * i], py = pts[3 * i + 1], pz = pts[3 * i + 2];
     int abortIdx = 0;
@@ -185,36 +217,45 @@ __global__ void __launch_bounds__(kListThreads) kSplatCount(const float *__restr
     }
     abortAt[i] = abortIdx;
     if (abortIdx == 0) continue;
+    bool hashed = HASH && !h.isFull();
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       if (sl[k] < 0) continue;
-      const int p = hashPlace<true>(h, sl[k]);
-      if (p >= 0) atomicAdd(&h.val[p], 1);
-      else atomicAdd(&cnt[sl[k]], 1);
+      const int p = hashed ? hashPlace<true>(h, sl[k]) : -1;
+      if (p >= 0) {
+        atomicAdd(&h.val[p], 1);
+      } else {
+        if (hashed) h.full = 1;
+        hashed = false;
+        atomicAdd(&cnt[sl[k]], 1);
+      }
     }
   }
+  if (!HASH) return;
   __syncthreads();
-  for (int i = threadIdx.x; i < kHashSize; i += kListThreads)
+  for (int i = threadIdx.x; i < kHashSize; i += NT)
     if (h.key[i] >= 0) atomicAdd(&cnt[h.key[i]], h.val[i]);
 }
 
 // Pass 2: the particle's index into the list of every value block it touches
 // (list of slot s: entries[off[s] .. off[s+1]-1], in no particular order).  The CTA counts
-// its particles per block, reserves a run of each list, and fills it.
-__global__ void __launch_bounds__(kListThreads) kSplatScatter(const float *__restrict__ pts, int64_t n, int ppt,
+// its particles per block, reserves a run of each list, and fills it (HASH), or takes every
+// position by itself.  *chunk: the list entries that a CTA of the third pass takes.
+template <int NT, bool HASH>
+__global__ void __launch_bounds__(NT) kSplatScatter(const float *__restrict__ pts, int64_t n, int ppt,
                                                               SplatGeom g, const int32_t *__restrict__ slot,
                                                               const int32_t *__restrict__ abortAt,
                                                               const int64_t *__restrict__ off,
                                                               int32_t *__restrict__ cursor,
-                                                              int32_t *__restrict__ entries) {
+                                                              int32_t *__restrict__ entries, int64_t nAct, ChunkRule rule,
+                                                              int *__restrict__ chunk) {
   __shared__ BlockHash h;
   __shared__ int run[kHashSize];  // the CTA's first position in a block's list
-  hashClear(h);
-  __syncthreads();
-  const int64_t first = (int64_t)blockIdx.x * ppt * kListThreads + threadIdx.x;
-  auto forBlocks = [&](auto f) {
-    for (int q = 0; q < ppt; q++) {
-      const int64_t i = first + (int64_t)q * kListThreads;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *chunk = rule.of(off[nAct]);
+  const int64_t first = (int64_t)blockIdx.x * ppt * NT + threadIdx.x;
+  auto forBlocks = [&](auto go, auto f) {
+    for (int q = 0; q < ppt && go(); q++) {
+      const int64_t i = first + (int64_t)q * NT;
       if (i >= n) break;
       if (abortAt[i] == 0) continue;
       SplatBox b;
@@ -226,21 +267,30 @@ __global__ void __launch_bounds__(kListThreads) kSplatScatter(const float *__res
         if (sl[k] >= 0) f(sl[k], (int32_t)i);
     }
   };
-  forBlocks([&](int sl, int32_t) {
-    const int p = hashPlace<true>(h, sl);
-    if (p >= 0) atomicAdd(&h.val[p], 1);
-  });
-  __syncthreads();
-  for (int i = threadIdx.x; i < kHashSize; i += kListThreads)
+  const auto always = [] { return true; };
+  if (HASH) {
+    hashClear(h);
+    __syncthreads();
+    forBlocks([&] { return !h.isFull(); }, [&](int sl, int32_t) {
+      const int p = hashPlace<true>(h, sl);
+      if (p >= 0) atomicAdd(&h.val[p], 1);
+      else h.full = 1;
+    });
+    __syncthreads();
+  }
+  if (!HASH || h.isFull()) {
+    forBlocks(always, [&](int sl, int32_t i) { entries[off[sl] + atomicAdd(&cursor[sl], 1)] = i; });
+    return;
+  }
+  for (int i = threadIdx.x; i < kHashSize; i += NT)
     if (h.key[i] >= 0) {
       run[i] = atomicAdd(&cursor[h.key[i]], h.val[i]);
       h.val[i] = 0;
     }
   __syncthreads();
-  forBlocks([&](int sl, int32_t i) {
+  forBlocks(always, [&](int sl, int32_t i) {  // every block has its place
     const int p = hashPlace<false>(h, sl);
-    const int at = p >= 0 ? run[p] + atomicAdd(&h.val[p], 1) : atomicAdd(&cursor[sl], 1);
-    entries[off[sl] + at] = i;
+    entries[off[sl] + run[p] + atomicAdd(&h.val[p], 1)] = i;
   });
 }
 
@@ -249,7 +299,7 @@ __global__ void __launch_bounds__(kListThreads) kSplatScatter(const float *__res
 // current values (init: FP32 channels, where the demo's splat takes the minimum
 // with what the channel holds) or from 1.0 (the FP32 staging of other storage
 // types, which the demo fills with 1.0 first), then one coalesced write of the
-// block.  Half a warp takes one particle at a time; its
+// block.  Half a warp or a warp (LANES) takes one particle at a time; its
 // lanes take the (y, z) rows of the box clipped to the block, skip rows already
 // outside the sphere (dz*dz + dy*dy exceeds it, and adding dx*dx >= 0 cannot lower
 // a float sum), and keep the voxels before the particle's abort index.
@@ -267,24 +317,18 @@ constexpr int splatThreads() { return 16 * BS; }
 template <int BS>
 constexpr int splatMinCtas() { return 1536 / splatThreads<BS>(); }
 
-// list entries a CTA takes
-template <int BS>
-constexpr int splatChunk() { return 32 * BS; }
-
-// Lanes that share a particle.  A box has 81 rows at the demo's radius, fewer where the block
+// LANES share a particle (the rule is at the launch).  A box has 81 rows at the demo's radius, fewer where the block
 // clips it, and every lane of a group works out the whole box: 8 / 16 / 32 lanes take 940 / 901
 // / 937 us for the splat of 768 k particles on 32^3 blocks, 4.07 / 4.05 / 4.26 ms for the 512^3
 // pipeline (smaller groups of a warp wait for its longest box).
-constexpr int kRowLanes = 16;
-
 // Entries e0 .. e1-1 of a block's list into the minima of its planes Z0 .. Z0+PZ-1.
 // Bound: issue (80% of the slots).
-template <int BS, int NZ>
+template <int BS, int NZ, int LANES>
 __device__ __forceinline__ void splatEntries(int *smin, const float *__restrict__ pts, const SplatGeom &g, int X0, int Y0,
                                              int Z0, const int32_t *__restrict__ abortAt,
                                              const int32_t *__restrict__ entries, int64_t e0, int64_t e1) {
   constexpr int RS = BS + 1, PZ = BS / NZ;
-  const int lane = threadIdx.x % kRowLanes, group = threadIdx.x / kRowLanes, nGroups = blockDim.x / kRowLanes;
+  const int lane = threadIdx.x % LANES, group = threadIdx.x / LANES, nGroups = blockDim.x / LANES;
   for (int64_t e = e0 + group; e < e1; e += nGroups) {
     const int i = entries[e];
     const float px = pts[3 * (int64_t)i], py = pts[3 * (int64_t)i + 1], pz = pts[3 * (int64_t)i + 2];
@@ -297,11 +341,11 @@ __device__ __forceinline__ void splatEntries(int *smin, const float *__restrict_
     const int cz1 = max(b.iz1, Z0), cz2 = min(b.iz2, Z0 + PZ - 1);
     const int cny = cy2 - cy1 + 1, cnz = cz2 - cz1 + 1;
     if (cx2 < cx1 || cny <= 0 || cnz <= 0) continue;
-    // the lane's rows: row = lane + kRowLanes k, decoded as (row % cny, row / cny) through an
+    // the lane's rows: row = lane + LANES k, decoded as (row % cny, row / cny) through an
     // approximate reciprocal (row < 34^2 and cny <= 33: the quotient's fraction stays
     // at least 1/(2 cny) away from an integer, so the truncation is exact)
     const float rcny = __frcp_rn((float)cny);
-    for (int row = lane; row < cny * cnz; row += kRowLanes) {
+    for (int row = lane; row < cny * cnz; row += LANES) {
       const int qz = (int)(((float)row + 0.5f) * rcny);
       const int iy = cy1 + row - qz * cny, iz = cz1 + qz;
       const float dz = __fsub_rn((float)iz, b.z0), dy = __fsub_rn((float)iy, b.y0);
@@ -336,30 +380,38 @@ __device__ __forceinline__ void splatEntries(int *smin, const float *__restrict_
 // CTA that took the longest list alone ran while the other SMs had finished: the SMs were
 // active 40% of the launch on the 512^3 workload (4.36 ms).  A longer list's other chunks
 // are queued for kSplatRest (0.34 + 1.53 ms).
-template <int BS, int NZ>
+template <int BS, int NZ, int LANES>
 __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatBlock(const float *__restrict__ pts, SplatGeom g,
                                                    const int32_t *__restrict__ active,
                                                    const int32_t *__restrict__ abortAt,
                                                    const int64_t *__restrict__ off,
                                                    const int32_t *__restrict__ entries, const float *init,
-                                                   float *dst, int *__restrict__ nRest, int2 *__restrict__ rest) {
-  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ, CH = splatChunk<BS>();
+                                                   float *dst, const int *__restrict__ chunk,
+                                                   int *__restrict__ nRest, int2 *__restrict__ rest) {
+  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ;
   extern __shared__ __align__(16) int smin[];
   __shared__ int restAt;
   const int sl = blockIdx.x / NZ, zp = blockIdx.x % NZ;
   const int bid = active[sl];
   const int X0 = (bid % g.nbx) * BS, Y0 = ((bid / g.nbx) % g.nby) * BS,
             Z0 = (int)(bid / ((int64_t)g.nbx * g.nby)) * BS + zp * PZ;  // this CTA's first plane
-  const int64_t e0 = off[sl], cnt = off[sl + 1] - e0;
-  const int more = zp == 0 && cnt > CH ? (int)((cnt - 1) / CH) : 0;
-  if (more && threadIdx.x == 0) restAt = atomicAdd(nRest, more);
+  const int64_t e0 = off[sl];
+  const int cnt = (int)(off[sl + 1] - e0), ch = *chunk;
   const int one = __float_as_int(1.0f);
+  if (cnt == 0) {  // no particle: the block keeps its values, or is 1
+    if (init) return;
+    int4 *o = reinterpret_cast<int4 *>(dst + (int64_t)sl * VPB + zp * VPP);
+    for (int v = threadIdx.x; v < VPP / 4; v += blockDim.x) o[v] = make_int4(one, one, one, one);
+    return;
+  }
   const float *in = init ? init + (int64_t)sl * VPB + zp * VPP : nullptr;
   for (int v = threadIdx.x; v < VPP; v += blockDim.x)
     smin[(v / BS) * RS + v % BS] = in ? __float_as_int(in[v]) : one;
+  const int more = zp == 0 && cnt > ch ? (cnt - 1) / ch : 0;
+  if (more && threadIdx.x == 0) restAt = atomicAdd(nRest, more);
   __syncthreads();
   for (int k = threadIdx.x; k < more; k += blockDim.x) rest[restAt + k] = make_int2(sl, k + 1);
-  splatEntries<BS, NZ>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, e0 + min(cnt, (int64_t)CH));
+  splatEntries<BS, NZ, LANES>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, e0 + min(cnt, ch));
   __syncthreads();
   float *out = dst + (int64_t)sl * VPB + zp * VPP;
   for (int v = threadIdx.x * 4; v < VPP; v += blockDim.x * 4) {
@@ -370,16 +422,16 @@ __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplat
 
 // The queued chunks: their minima are merged into the blocks that kSplatBlock has written
 // (integer minima of the bit patterns, as there).
-template <int BS, int NZ>
+template <int BS, int NZ, int LANES>
 __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatRest(const float *__restrict__ pts, SplatGeom g,
                                                    const int32_t *__restrict__ active,
                                                    const int32_t *__restrict__ abortAt,
                                                    const int64_t *__restrict__ off,
                                                    const int32_t *__restrict__ entries, int *dst,
-                                                   const int *__restrict__ nRest, const int2 *__restrict__ rest) {
-  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ, CH = splatChunk<BS>();
+                                                   const int *__restrict__ chunk, const int *__restrict__ nRest, const int2 *__restrict__ rest) {
+  constexpr int VPB = BS * BS * BS, RS = BS + 1, PZ = BS / NZ, VPP = BS * BS * PZ;
   extern __shared__ __align__(16) int smin[];
-  const int n = *nRest * NZ;
+  const int n = *nRest * NZ, ch = *chunk;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const int2 r = rest[w / NZ];
     const int sl = r.x, zp = w % NZ, bid = active[sl];
@@ -387,8 +439,8 @@ __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplat
               Z0 = (int)(bid / ((int64_t)g.nbx * g.nby)) * BS + zp * PZ;
     for (int v = threadIdx.x; v < VPP; v += blockDim.x) smin[(v / BS) * RS + v % BS] = 0x7fffffff;
     __syncthreads();
-    const int64_t e0 = off[sl] + (int64_t)r.y * CH;
-    splatEntries<BS, NZ>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, min(e0 + CH, off[sl + 1]));
+    const int64_t e0 = off[sl] + (int64_t)r.y * ch;
+    splatEntries<BS, NZ, LANES>(smin, pts, g, X0, Y0, Z0, abortAt, entries, e0, min(e0 + ch, off[sl + 1]));
     __syncthreads();
     int *out = dst + (int64_t)sl * VPB + zp * VPP;
     for (int v = threadIdx.x; v < VPP; v += blockDim.x) {
@@ -510,46 +562,76 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
   int32_t *abortAt = (int32_t *)scratch;
   int32_t *cnt = (int32_t *)(scratch + ((bAbort + 15) & ~size_t(15)));
   int32_t *cursor = (int32_t *)((char *)cnt + bCnt);
-  int *nRest = (int *)((char *)cursor + bCnt);
+  int *nRest = (int *)((char *)cursor + bCnt), *chunk = nRest + 1;
   int64_t *off = (int64_t *)((char *)nRest + 16);
   int2 *rest = (int2 *)((char *)off + ((bOff + 15) & ~size_t(15)));
   int32_t *entries = (int32_t *)((char *)rest + ((bRest + 15) & ~size_t(15)));
   // particles per thread of the list passes: more per CTA share its table, while the CTAs
   // still fill the chip
   const int ppt = n >= (int64_t)152 * 4 * kListThreads * 8 ? 8 : n >= (int64_t)152 * 4 * kListThreads * 2 ? 4 : 1;
-  const unsigned listGrid = gridFor(n, ppt * kListThreads);
+  // The table pays where a block has many particles; with few, and for the smallest calls, its
+  // set-up and flush cost more than they save.  Splat of FP16 blocks in us, table / none: 1 M
+  // particles on shells in 32^3 blocks (radius 4) 1040 / 1532, 100 k so 157 / 191, 10 k 69 / 66;
+  // 1 M in no order on 262 k blocks of 8^3 (radius 1) 670 / 627; 1 k on shells 51 / 45.
+  const bool hash = n >= 2048 && n >= 64 * nAct;
+  const unsigned listGrid = hash ? gridFor(n, ppt * kListThreads) : gridFor(n, kDirectThreads);
+  const int nz = ctx->bsx == 32 ? 2 : 1;
+  const int places = 152 * 1536 / (16 * ctx->bsx);
+  const ChunkRule rule{32 * ctx->bsx, places, nz, nz * nAct <= places / 2};
   int rc = MSBG_GPU_OK;
   auto run = [&]() -> int {
     MSBG_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * bCnt + 16, ctx->stream));
     if (n > 0) {
-      MSBG_LAUNCH(ctx, kSplatCount, listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt, cnt,
-                  (unsigned long long *)(ctx->dCounters + 1));
+      unsigned long long *aborted = (unsigned long long *)(ctx->dCounters + 1);
+      if (hash)
+        MSBG_LAUNCH(ctx, (kSplatCount<kListThreads, true>), listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt,
+                    cnt, aborted);
+      else
+        MSBG_LAUNCH(ctx, (kSplatCount<kDirectThreads, false>), listGrid, kDirectThreads, 0, dPts, n, 1, g, ctx->dSlot,
+                    abortAt, cnt, aborted);
     }
     int r = exclusiveScanCounts(ctx, cnt, nAct, off, off + nAct);
     if (r) return r;
     if (n > 0) {
-      MSBG_LAUNCH(ctx, kSplatScatter, listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt, off, cursor,
-                  entries);
+      if (hash)
+        MSBG_LAUNCH(ctx, (kSplatScatter<kListThreads, true>), listGrid, kListThreads, 0, dPts, n, ppt, g, ctx->dSlot, abortAt,
+                    off, cursor, entries, nAct, rule, chunk);
+      else
+        MSBG_LAUNCH(ctx, (kSplatScatter<kDirectThreads, false>), listGrid, kDirectThreads, 0, dPts, n, 1, g, ctx->dSlot,
+                    abortAt, off, cursor, entries, nAct, rule, chunk);
     }
     const float *init = c.storage == MSBG_GPU_F32 ? dst : nullptr;
-    auto blocks = [&](auto bsC, auto nzC) -> int {
-      constexpr int BS = decltype(bsC)::value, NZ = decltype(nzC)::value, smem = splatSmemWords<BS, NZ>() * 4;
+    auto blocks = [&](auto bsC, auto nzC, auto lanesC) -> int {
+      constexpr int BS = decltype(bsC)::value, NZ = decltype(nzC)::value, LANES = decltype(lanesC)::value;
+      constexpr int smem = splatSmemWords<BS, NZ>() * 4;
+      const auto block = kSplatBlock<BS, NZ, LANES>;
+      const auto restKern = kSplatRest<BS, NZ, LANES>;
       if (smem > 48 * 1024) {
         static SmemOptIn optInBlock, optInRest;
-        MSBG_CUDA(ctx, optInBlock((const void *)kSplatBlock<BS, NZ>, smem));
-        MSBG_CUDA(ctx, optInRest((const void *)kSplatRest<BS, NZ>, smem));
+        MSBG_CUDA(ctx, optInBlock((const void *)block, smem));
+        MSBG_CUDA(ctx, optInRest((const void *)restKern, smem));
       }
-      MSBG_LAUNCH(ctx, (kSplatBlock<BS, NZ>), (unsigned)(NZ * nAct), splatThreads<BS>(), smem, dPts, g, ctx->dActive,
-                  abortAt, off, entries, init, dst, nRest, rest);
-      if (n > splatChunk<BS>())
-        MSBG_LAUNCH(ctx, (kSplatRest<BS, NZ>), 152 * splatMinCtas<BS>(), splatThreads<BS>(), smem, dPts, g, ctx->dActive,
-                    abortAt, off, entries, (int *)dst, nRest, rest);
+      MSBG_LAUNCH(ctx, block, (unsigned)(NZ * nAct), splatThreads<BS>(), smem, dPts, g, ctx->dActive, abortAt, off,
+                  entries, init, dst, chunk, nRest, rest);
+      if (n > rule.leastOf(8 * n))  // a list may be longer than a chunk
+        MSBG_LAUNCH(ctx, restKern, (unsigned)std::min<int64_t>(places, nz * (8 * n / rule.least + 1)), splatThreads<BS>(), smem, dPts, g, ctx->dActive, abortAt,
+                    off, entries, (int *)dst, chunk, nRest, rest);
       return MSBG_GPU_OK;
     };
     using std::integral_constant;
-    if (ctx->bsx == 32) return blocks(integral_constant<int, 32>{}, integral_constant<int, 2>{});
-    if (ctx->bsx == 16) return blocks(integral_constant<int, 16>{}, integral_constant<int, 1>{});
-    return blocks(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+    const int edge = (int)(2.0f * g.rScan) + 1;
+    // Whole warps for boxes of 128 rows and more (the half warps of a warp wait for the longer
+    // of two clipped boxes) and where a block has fewer particles than warps.  32^3 blocks, half /
+    // whole warps, us: 1 M particles on shells, radius 2.5 557 / 667, radius 4 1038 / 1066; 100 k,
+    // radius 4 156 / 163, radius 6 313 / 291, radius 10 971 / 766; 10 k in no order, radius 4 169 /
+    // 159, radius 2.5 152 / 150.
+    const bool wide = edge * edge >= 128 || n <= nAct * (ctx->bsx / 2);
+    auto sized = [&](auto lanesC) -> int {
+      if (ctx->bsx == 32) return blocks(integral_constant<int, 32>{}, integral_constant<int, 2>{}, lanesC);
+      if (ctx->bsx == 16) return blocks(integral_constant<int, 16>{}, integral_constant<int, 1>{}, lanesC);
+      return blocks(integral_constant<int, 8>{}, integral_constant<int, 1>{}, lanesC);
+    };
+    return wide ? sized(integral_constant<int, 32>{}) : sized(integral_constant<int, 16>{});
   };
   rc = run();
   cudaFreeAsync(scratch, ctx->stream);
