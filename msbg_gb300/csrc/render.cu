@@ -41,6 +41,8 @@
 // one that stepping gives, bit for bit.  1280x720 of a 48-cluster crop of the 4096^3 FP16
 // layout: 60.3 ms stepping, 1.81 ms so.  Bound now: issue and instruction fetch (34% of
 // issue slots, 24 of 32 lanes active), the rays of a warp parting at cell faces.
+#include <type_traits>
+
 #include "interp_common.cuh"
 
 namespace msbg {
@@ -127,9 +129,13 @@ __device__ __forceinline__ bool axisAhead(const Axis &a, bool down, long long n,
   nb = a.b + n * a.j;
   return a.fast && ((nb ^ a.b) >> 52) == 0 && !(down && (nb & kMant) == 0);
 }
+// FEW: the rounded sum itself; j is then derived before a jump.
+template <bool FEW>
 __device__ __forceinline__ void axisStep(Axis &a, bool down, double inc) {
   long long nb;
-  if (axisAhead(a, down, 1, nb)) {
+  if (FEW) {
+    a.b = __double_as_longlong(__dadd_rn(__longlong_as_double(a.b), inc));
+  } else if (axisAhead(a, down, 1, nb)) {
     a.b = nb;
   } else {
     a.b = __double_as_longlong(__dadd_rn(__longlong_as_double(a.b), inc));
@@ -137,9 +143,10 @@ __device__ __forceinline__ void axisStep(Axis &a, bool down, double inc) {
   }
 }
 // __double2float_rn of a position's pattern
+template <bool FEW>
 __device__ __forceinline__ float patternToFloat(long long b) {
   const int e = (int)((b >> 52) & 0x7ff);
-  if (b < 0 || e <= 1023 - 126 || e >= 1023 + 126) return __double2float_rn(__longlong_as_double(b));
+  if (FEW || b < 0 || e <= 1023 - 126 || e >= 1023 + 126) return __double2float_rn(__longlong_as_double(b));
   const unsigned long long f = (unsigned long long)(b - ((1023ll - 127) << 52));
   return __uint_as_float((uint32_t)((f + 0x0fffffffull + ((f >> 29) & 1)) >> 29));
 }
@@ -231,8 +238,14 @@ __device__ RV gradient(const RenderArgs &a, RV p) {
   return {-(double)gx, -(double)gy, -(double)gz};
 }
 
-template <typename T>
-__global__ void __launch_bounds__(128, 6) kRender(RenderArgs a) {
+// FEW: pictures whose CTAs all fit the chip at four an SM.  Their rays are as long as the steps'
+// latency, not as the FP64 pipe or issue take, and an FP64 sum is shorter than the integer step
+// (and its spills at 80 registers): full layouts of 16^3 blocks that no ray hits, 48x27 563 us
+// with integer steps, 469 so, 434 before the integer steps; 320x180 511 / 442 / 479; 480x270
+// (1020 CTAs) 679 / 678 / 750; 1280x720 2782 / 3207 / 4197.
+constexpr unsigned kFewCtas = 152 * 4;
+template <typename T, bool FEW>
+__global__ void __launch_bounds__(128, FEW ? 4 : 6) kRender(RenderArgs a) {
   // a warp takes 8x4 pixels, whose rays stay together longer than a 16x2 row pair's
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7), y = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
@@ -257,7 +270,7 @@ __global__ void __launch_bounds__(128, 6) kRender(RenderArgs a) {
     ax[k].b = __double_as_longlong(start[k]);
     zero[k] = (__double_as_longlong(incv[k]) << 1) == 0;
     down[k] = __double2hiint(incv[k]) < 0 && !zero[k];
-    axisDerive(ax[k], incv[k]);
+    if (!FEW) axisDerive(ax[k], incv[k]);
     q[k] = __fmul_rn(a.res, __double2float_rn(start[k]));
     dirV[k] = a.res * (float)incv[k];
     invDir[k] = dirV[k] != 0.0f ? 1.0f / dirV[k] : 0.0f;
@@ -296,8 +309,9 @@ __global__ void __launch_bounds__(128, 6) kRender(RenderArgs a) {
         float q2[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
+          if (FEW) axisDerive(ax[k], incv[k]);
           in = axisAhead(ax[k], down[k], steps, nb[k]) && in;
-          q2[k] = __fmul_rn(a.res, patternToFloat(nb[k]));
+          q2[k] = __fmul_rn(a.res, patternToFloat<FEW>(nb[k]));
           const float f = floorf(q2[k]);
           in = in && f >= (float)lo[k] && f < (float)hi[k];
         }
@@ -313,8 +327,9 @@ __global__ void __launch_bounds__(128, 6) kRender(RenderArgs a) {
     }
     // Inside a value block the next kAhead steps are evaluated together, so that their
     // gathers overlap; they are then looked at in order, as single steps are.  Two: one
-    // takes 2.00 ms, four 2.58 (instruction fetch), on the view named at the top.
-    constexpr int kAhead = 2;
+    // takes 2.00 ms, four 2.58 (instruction fetch), on the view named at the top.  FEW: one, as
+    // two lengthen the step (48x27 as above 1.30x against 1.16x with integer steps).
+    constexpr int kAhead = FEW ? 1 : 2;
     const int nAhead = where == kValue ? kAhead : 1;
     Axis at1[3] = {ax[0], ax[1], ax[2]};
     long long pb[kAhead][3];
@@ -327,9 +342,9 @@ __global__ void __launch_bounds__(128, 6) kRender(RenderArgs a) {
       if (i >= nAhead) continue;
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        axisStep(at1[k], down[k], incv[k]);
+        axisStep<FEW>(at1[k], down[k], incv[k]);
         pb[i][k] = at1[k].b;
-        q[k] = __fmul_rn(a.res, patternToFloat(at1[k].b));
+        q[k] = __fmul_rn(a.res, patternToFloat<FEW>(at1[k].b));
         const float f = floorf(q[k]);
         gone[i] |= (f < 0.0f && (down[k] || zero[k])) || (f > (float)(s[k] - 1) && !down[k]);
       }
@@ -433,11 +448,15 @@ extern "C" int msbg_gpu_render(msbg_gpu_ctx *ctx, int chan, int width, int heigh
               n16y, ctx->dOccupancy, g16);
   a.occ = {ctx->dOccupancy, g16, n4x, n4y, n16x, n16y};
   const dim3 grid((unsigned)((width + 15) / 16), (unsigned)((height + 7) / 8));
-  switch (c.storage) {
-    case MSBG_GPU_F32: MSBG_LAUNCH(ctx, kRender<float>, grid, 128, 0, a); break;
-    case MSBG_GPU_F16: MSBG_LAUNCH(ctx, kRender<__half>, grid, 128, 0, a); break;
-    case MSBG_GPU_U16: MSBG_LAUNCH(ctx, kRender<uint16_t>, grid, 128, 0, a); break;
-    default: return fail(ctx, MSBG_GPU_ERR_UNSUPPORTED, "render: FP64 channels are not supported");
-  }
-  return MSBG_GPU_OK;
+  auto launch = [&](auto few) -> int {
+    constexpr bool FEW = decltype(few)::value;
+    switch (c.storage) {
+      case MSBG_GPU_F32: MSBG_LAUNCH(ctx, (kRender<float, FEW>), grid, 128, 0, a); break;
+      case MSBG_GPU_F16: MSBG_LAUNCH(ctx, (kRender<__half, FEW>), grid, 128, 0, a); break;
+      case MSBG_GPU_U16: MSBG_LAUNCH(ctx, (kRender<uint16_t, FEW>), grid, 128, 0, a); break;
+      default: return fail(ctx, MSBG_GPU_ERR_UNSUPPORTED, "render: FP64 channels are not supported");
+    }
+    return MSBG_GPU_OK;
+  };
+  return (int64_t)grid.x * grid.y <= kFewCtas ? launch(std::true_type{}) : launch(std::false_type{});
 }
