@@ -320,8 +320,8 @@ int tailBuildTables(msbg_gpu_ctx *ctx, PoissonState *ps) {
 }
 
 // The V-cycle of the levels from l in one launch.  *done: whether this form takes them: every
-// one is relaxed pointwise, the coarsest is solved by its inverse, and level l is small
-// enough that a sweep costs less than the launch it would otherwise be.
+// one is relaxed pointwise, the coarsest is solved by its inverse, and level l has at most
+// kTailMaxCells cells.
 template <typename V>
 int coarseTail(msbg_gpu_ctx *ctx, PoissonState *ps, const PrecSet &P, size_t l, bool *done) {
   *done = false;
