@@ -18,8 +18,8 @@ FP32 arithmetic, 8-color in-place mean-curvature-flow sweeps (laplTyp 4).
   bounded sample of the same workload.
 
 ``--impl reference`` times the reference's CPU implementation of the path on
-the host cores instead: the reference library built from its sources where it
-compiles (x86-64), else the CPU restatement of it (aarch64 hosts).
+the host cores instead: the reference library built from its sources, on x86-64
+hosts that have them.  Elsewhere it says that it is unavailable, and why.
 Multi-GPU: the path does not shard here ("replicas only"); N ranks each run the
 full workload and ``value`` is the sum over ranks.
 """
@@ -208,46 +208,41 @@ def cpu_sample(spec: dict, pts: np.ndarray, target_sec: float = 10.0, max_blocks
 # reference arm
 # ------------------------------------------------------------------------------------
 def run_reference(args, spec, dist: Dist):
+    """The reference library's own sweep timing, on the host it compiles on; no number of this
+    project's code takes its place elsewhere."""
     if dist.rank != 0:
         return
-    pts = W.make_points(spec, 1 if spec is W.SURFACE_512 else 2)
     arch = platform.machine()
     ref_driver = os.path.join(ROOT, "oracle", "_ref", "msbg_ref_driver")
-    kind = "port"
-    vals = []
-    desc = ""
+    if arch not in ("x86_64", "AMD64"):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          f"the reference's CPU code is x86 SIMD and does not compile on {arch}"}), flush=True)
+        return
+    if not os.path.isfile(ref_driver):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "oracle/_ref/msbg_ref_driver is not built (the reference's sources are not here)"}),
+              flush=True)
+        return
+    pts = W.make_points(spec, 1 if spec is W.SURFACE_512 else 2)
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle_io as O
     threads = os.cpu_count() or 1
-    if arch in ("x86_64", "AMD64") and os.path.isfile(ref_driver):
-        # the reference library itself on a cropped sample (its MCF sweep timing)
-        sys.path.insert(0, os.path.join(ROOT, "oracle"))
-        import oracle_io as O
-        kind = "reference"
-        res = 1024 if spec["res"] > 1024 else spec["res"]
-        sub = pts[(pts < res - 1).all(axis=1)]
-        for _ in range(args.warmup + args.steps):
-            job = O.SurfaceJob(res, res, res, spec["bsx"], sub, chan=O.CHAN_U16, n_iter=4, dt=0.1,
-                               n_threads=threads)
-            r = O.run_reference_surface(job)
-            vals.append(r.n_active * spec["bsx"] ** 3 * 4 / r.times["pde"])
-        vals = vals[args.warmup:]
-        desc = (f"reference applyChannelPdeFast<uint16> MCF, 4 iterations over the level-0 blocks of "
-                f"the workload's points inside a {res}^3 crop")
-        dtype = "u16 storage / f32 math"
-    else:
-        for i in range(args.warmup + args.steps):
-            v, desc, threads = cpu_sample(spec, pts, target_sec=8.0)
-            vals.append(v)
-        vals = vals[args.warmup:]
-        desc = "reference CPU path unavailable on this host (x86 SIMD); " + desc
-        dtype = "f16 storage / f32 math" if spec["storage"] == "f16" else "f32"
-    value = float(np.median(vals))
+    res = 1024 if spec["res"] > 1024 else spec["res"]
+    sub = pts[(pts < res - 1).all(axis=1)]
+    vals = []
+    for _ in range(args.warmup + args.steps):
+        job = O.SurfaceJob(res, res, res, spec["bsx"], sub, chan=O.CHAN_U16, n_iter=4, dt=0.1, n_threads=threads)
+        r = O.run_reference_surface(job)
+        vals.append(r.n_active * spec["bsx"] ** 3 * 4 / r.times["pde"])
+    value = float(np.median(vals[args.warmup:]))
     line = {
         "impl": "reference", "metric": "voxel-updates/s (MCF sweeps)", "value": value,
         "unit": "voxel-updates/s", "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
-        "higher_is_better": True, "dtype": dtype, "data": "synthetic",
+        "higher_is_better": True, "dtype": "u16 storage / f32 math", "data": "synthetic",
         "config": {"workload": spec["name"]},
-        "cpu_baseline": {"value": value, "unit": "voxel-updates/s", "cores": threads, "kind": kind,
-                         "sample": desc},
+        "cpu_baseline": {"value": value, "unit": "voxel-updates/s", "cores": threads, "kind": "reference",
+                         "sample": "reference applyChannelPdeFast<uint16> MCF, 4 iterations over the level-0 blocks of "
+                                   f"the workload's points inside a {res}^3 crop"},
         "e2e": {"value": value, "unit": "voxel-updates/s", "h2d_bytes_per_step": 0,
                 "d2h_bytes_per_step": 0},
     }
