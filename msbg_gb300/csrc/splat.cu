@@ -144,21 +144,21 @@ __device__ __forceinline__ bool boxSlots(const SplatGeom &g, const SplatBox &b, 
 }
 
 // List entries that a CTA of the third pass takes: an eighth of an even share of all entries
-// over the CTAs that the chip holds (places), and at least 32 bs: without the share, 3 M
-// particles in no order split every list in two (32^3 blocks, radius 4: 2.99 ms, 2.37 so).
-// With fewer entries than two such chunks a place, four times that: a split list's chunks wait
-// for the first ones of all, which pays only where the blocks leave most places empty (100 k
-// particles in a ball, 32^3 blocks, 32 bs / four times that: radius 4 220 / 175 us, radius 10
-// 1085 / 907; the 64^3 frame's 38 blocks 1223 us a frame with four times that, 1183 so).
+// over the CTAs that the chip holds (places), and at least 32 bs.  Without the share, 3 M
+// particles in no order split every list in two (32^3 blocks, radius 4: 2.99 ms, 2.37 so).  Four
+// times as many at least costs scenes whose particles crowd into a few blocks more (172 k on 56
+// spheres, 1805 blocks of 16^3: 492 us, 280 so) than it saves where the lists are even (100 k in
+// a ball, 32^3 blocks, radius 4: 175 us, 220 so; radius 10 907 and 1085).  whole: so few particles
+// over so many blocks that the second launch is left out.
 struct ChunkRule {
   int least, places, nz;
-  bool fewBlocks;
-  __host__ __device__ int of(int64_t total) const {
-    const int64_t share = total * nz / places;
-    if (share < 2 * least) return fewBlocks ? least : 4 * least;
-    return share / 8 < least ? least : (int)(share / 8);
+  bool whole;
+  ChunkRule(int bs, int64_t nAct, int64_t n)
+      : least(32 * bs), places(152 * 1536 / (16 * bs)), nz(bs == 32 ? 2 : 1),
+        whole(n <= least || (n <= 4 * least && nz * nAct > places / 2)) {}
+  __device__ int of(int64_t total) const {
+    return whole ? 4 * least : (int)max((int64_t)least, total * nz / (8 * places));
   }
-  int leastOf(int64_t upTo) const { return upTo * nz / places < 2 * least ? of(0) : least; }  // of any total
 };
 
 // Pass 1.  Valid particles (the marking loop's domain tests, src/msbg_demo.cpp:358-360, and
@@ -571,13 +571,12 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
   const int ppt = n >= (int64_t)152 * 4 * kListThreads * 8 ? 8 : n >= (int64_t)152 * 4 * kListThreads * 2 ? 4 : 1;
   // The table pays where a block has many particles; with few, and for the smallest calls, its
   // set-up and flush cost more than they save.  Splat of FP16 blocks in us, table / none: 1 M
-  // particles on shells in 32^3 blocks (radius 4) 1040 / 1532, 100 k so 157 / 191, 10 k 69 / 66;
+  // particles on shells in 32^3 blocks (radius 4) 1040 / 1532, 100 k so 157 / 191, 10 k (33 a
+  // block) 69 / 66;
   // 1 M in no order on 262 k blocks of 8^3 (radius 1) 670 / 627; 1 k on shells 51 / 45.
-  const bool hash = n >= 2048 && n >= 64 * nAct;
+  const bool hash = n >= 2048 && n >= 48 * nAct;
   const unsigned listGrid = hash ? gridFor(n, ppt * kListThreads) : gridFor(n, kDirectThreads);
-  const int nz = ctx->bsx == 32 ? 2 : 1;
-  const int places = 152 * 1536 / (16 * ctx->bsx);
-  const ChunkRule rule{32 * ctx->bsx, places, nz, nz * nAct <= places / 2};
+  const ChunkRule rule(ctx->bsx, nAct, n);
   int rc = MSBG_GPU_OK;
   auto run = [&]() -> int {
     MSBG_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * bCnt + 16, ctx->stream));
@@ -613,9 +612,9 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
       }
       MSBG_LAUNCH(ctx, block, (unsigned)(NZ * nAct), splatThreads<BS>(), smem, dPts, g, ctx->dActive, abortAt, off,
                   entries, init, dst, chunk, nRest, rest);
-      if (n > rule.leastOf(8 * n))  // a list may be longer than a chunk
-        MSBG_LAUNCH(ctx, restKern, (unsigned)std::min<int64_t>(places, nz * (8 * n / rule.least + 1)), splatThreads<BS>(), smem, dPts, g, ctx->dActive, abortAt,
-                    off, entries, (int *)dst, chunk, nRest, rest);
+      if (!rule.whole)
+        MSBG_LAUNCH(ctx, restKern, (unsigned)std::min<int64_t>(rule.places, NZ * (8 * n / rule.least + 1)),
+                    splatThreads<BS>(), smem, dPts, g, ctx->dActive, abortAt, off, entries, (int *)dst, chunk, nRest, rest);
       return MSBG_GPU_OK;
     };
     using std::integral_constant;

@@ -1,7 +1,7 @@
 """The splat's launch rules against the CPU restatement, bit for bit: whole warps per particle
-(wide boxes; fewer particles than a block has warps), and lists split in longer chunks on
-layouts whose blocks fill the chip but hold few particles (a list just below, at and above four
-chunks, and several such chunks long)."""
+(wide boxes; fewer particles than a block has warps), and one block's list on layouts whose
+blocks fill the chip, just below, at and above the count from which lists are split, and many
+chunks long."""
 from __future__ import annotations
 
 import numpy as np
@@ -52,7 +52,7 @@ def test_long_lists_on_wide_layouts(gpulib, port, bsx, nblk, storage, count):
     res = nblk * bsx
     c = (np.arange(nblk) + 0.5) * bsx
     every = np.stack(np.meshgrid(c, c, c), -1).reshape(-1, 3)  # one particle in every block
-    n = 4 * 32 * bsx + count - 1
+    n = 4 * 32 * bsx + count - nblk ** 3  # particles in all: those in every block are part of the count
     spot = 3.5 * bsx + rng.uniform(-0.1, 0.1, (n, 3)) * bsx
     n_act = _check(gpulib, port, np.concatenate([spot, every]), res, bsx, storage, 1.5, 1.0)
     assert n_act == nblk ** 3 and n_act * (2 if bsx == 32 else 1) > 152 * 1536 // (16 * bsx) // 2
