@@ -48,8 +48,9 @@ from msbg_gb300 import workloads as W  # noqa: E402
 OPT8 = 1 << 29
 MCF8 = -(4 + OPT8)
 JAC8 = -(17 + OPT8)  # Jacobi diffusion (phi + dt sum f_i) / (1 + 6 dt), 8-colour in place
-# DRAM bytes (read + write) of one sweep launch of the 4096^3 workload, from an ncu
-# capture of the sweep kernel on this workload (mean of 8 launches)
+# DRAM bytes (read + write) of one sweep launch of the 4096^3 workload, from an ncu capture of
+# the sweep kernel on this workload (mean of 8 launches); the kernel has since changed what it
+# does with the staged tile, not what it stages (same bytes on the 96-cluster crop)
 SWEEP_TRAFFIC_4096 = 2.63e9
 
 
@@ -509,7 +510,7 @@ def run_gpu(args, spec, dist: Dist):
         "restriction": restriction,
         "g2p": g2p,
         "field_error_vs_fp64": field_error,
-        "splat": {"kernel": "kSplatCount + kSplatScatter + kSplatBlock (particles sorted into per-block "
+        "splat": {"kernel": "kSplatCount + kSplatScatter + kSplatBlock + kSplatRest (particles sorted into per-block "
                             "lists; blocks of 32^3 split into two CTAs by z-half, smaller blocks one CTA; "
                             "minimum in shared memory)", "ms_per_call": splat_ms,
                   "particles_per_s": n * dist.world / (splat_ms / 1e3)},

@@ -88,11 +88,9 @@ __device__ __forceinline__ bool splatBox(const SplatGeom &g, float px, float py,
 // come one after another, so thousands of atomics at a time met on the same few hundred
 // addresses (2.05 M particles of the 512^3 workload: 346 us to count, 357 us to scatter).
 // A CTA therefore sums its particles' blocks in a hash table in shared memory and goes to
-// the global counters once per block (33 and 62 us).  A block that finds no place within
-// kHashProbes goes to the global counter directly; whether it has a place is the same for
-// every thread and both passes over the particles, since places are never given back.
-// Once half the places are taken, the CTA goes on without the table: most of its blocks come
-// once (particles in no order, or spread over a volume).
+// the global counters once per block (35 and 65 us).  Places are never given back.  Once half
+// of them are taken, or a block finds none within kHashProbes, the CTA goes on without the table
+// (full): most of its blocks come once (particles in no order, or spread over a volume).
 constexpr int kListThreads = 512, kHashSize = 2048, kHashProbes = 16;
 constexpr int kDirectThreads = 256;  // of the forms without the table
 struct BlockHash {
@@ -379,7 +377,7 @@ __device__ __forceinline__ void splatEntries(int *smin, const float *__restrict_
 // numbers of particles (a small sphere's 32,000 particles lie in a few dozen blocks), and a
 // CTA that took the longest list alone ran while the other SMs had finished: the SMs were
 // active 40% of the launch on the 512^3 workload (4.36 ms).  A longer list's other chunks
-// are queued for kSplatRest (0.34 + 1.53 ms).
+// are queued for kSplatRest (0.43 + 1.27 ms).
 template <int BS, int NZ, int LANES>
 __global__ void __launch_bounds__(splatThreads<BS>(), splatMinCtas<BS>()) kSplatBlock(const float *__restrict__ pts, SplatGeom g,
                                                    const int32_t *__restrict__ active,
@@ -567,13 +565,13 @@ int splatRun(msbg_gpu_ctx *ctx, const float *dPts, int64_t n, float rParticle, f
   int2 *rest = (int2 *)((char *)off + ((bOff + 15) & ~size_t(15)));
   int32_t *entries = (int32_t *)((char *)rest + ((bRest + 15) & ~size_t(15)));
   // particles per thread of the list passes: more per CTA share its table, while the CTAs
-  // still fill the chip
+  // still fill the chip.  Splat on 2,100 blocks of 16^3 in us, 1 / 4 / 8 a thread: 300 k particles
+  // 108 / 114 / 127, 700 k 193 / 195 / 205, 1.5 M 305 / 297 / 304, 3 M 536 / 517 / 520, 10 M 1674 / 1596 / 1596.
   const int ppt = n >= (int64_t)152 * 4 * kListThreads * 8 ? 8 : n >= (int64_t)152 * 4 * kListThreads * 2 ? 4 : 1;
   // The table pays where a block has many particles; with few, and for the smallest calls, its
   // set-up and flush cost more than they save.  Splat of FP16 blocks in us, table / none: 1 M
   // particles on shells in 32^3 blocks (radius 4) 1040 / 1532, 100 k so 157 / 191, 10 k (33 a
-  // block) 69 / 66;
-  // 1 M in no order on 262 k blocks of 8^3 (radius 1) 670 / 627; 1 k on shells 51 / 45.
+  // block) 69 / 66, 1 k 51 / 45; 1 M in no order on 262 k blocks of 8^3 (radius 1) 670 / 627.
   const bool hash = n >= 2048 && n >= 48 * nAct;
   const unsigned listGrid = hash ? gridFor(n, ppt * kListThreads) : gridFor(n, kDirectThreads);
   const ChunkRule rule(ctx->bsx, nAct, n);

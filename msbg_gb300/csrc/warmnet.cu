@@ -673,11 +673,11 @@ __global__ void __launch_bounds__(kTcThreads, BS1 == 16 ? 3 : 2) kConvTcStaged(W
 // backward convolutions on level-1 blocks of edge 16 and 8 (CUDA cores; FP32)
 // ---------------------------------------------------------------------------------
 // Both gradients are FP32 contractions over 27 taps (their operands are FP32, so the BF16
-// tensor path of the forward pass would lose bits).  The bound is the FP32 pipe: 4.6 GFMA
-// a 16-16 layer on 663 k cells, 115 us at 128 lanes per SM and clock.  The forms below
+// tensor path of the forward pass would lose bits).  The bound is the FP32 pipe: 4.8 GFMA
+// a 16-16 layer on 696 k cells, 119 us at 128 lanes per SM and clock.  The forms below
 // stage a tile of 512 cells with its halo in shared memory once and keep enough products
 // per shared-memory load (11 to 24) for the packed FMAs to be the limit.  Measured on that
-// layout: kBwdData 223 us and kBwdWeight 241 us for a 16-16 layer (52% and 48% of the FP32
+// layout: kBwdData 223 us and kBwdWeight 241 us for a 16-16 layer (53% and 49% of the FP32
 // pipe); a step's three data and four weight launches 495 and 438 us, against 2703 and
 // 2854 us with the neighbours read from global memory per tap (the forms below, kept for
 // blocks of edge 4); the whole loss and gradient 6.02 -> 1.57 ms.
